@@ -7,11 +7,12 @@
 //                            matrix, viewport (Tracker.cpp:603-634) and crop;
 //   k_setup       1 block:  the tile layout of every crop, with prefix sums;
 //   k_tile_map    grid-stride: each ray and view tile's (item, view);
-//   k_ray         persistent: 16x16-ray tiles pulled from an atomic queue,
-//                            DRRs written to a packed buffer; rays with a
-//                            sample within rounding of the cutoff are listed;
-//   k_ray_fix     a warp per listed tile: its marked rays marched again
-//                            with exact cutoff decisions;
+//   k_ray         persistent: a warp per beam of 32 rays from an atomic
+//                            queue, DRRs written to a packed buffer; rays
+//                            with a sample within rounding of the cutoff are
+//                            marked, their beams listed;
+//   k_ray_fix     a warp per listed beam: its marked rays marched again with
+//                            exact cutoff decisions;
 //   k_view        persistent: 48x48 output tiles pulled from a queue; each
 //                            stages DRR and radiograph regions with the chain's
 //                            halo in shared memory, runs both filter chains,
@@ -31,6 +32,7 @@
 #include <vector>
 
 #include "asc_internal.cuh"
+#include "asc_rays.cuh"
 
 namespace asc {
 const void* image_data(asc_image im, int* w, int* h, int* bps);
@@ -52,9 +54,6 @@ constexpr int MAX_FILTERS = 8;
 #endif
 constexpr int VT = ASC_VT;   // k_view output tile edge
 constexpr int VNT = 256;     // k_view threads per block
-constexpr int RTX = 16, RTY = 16;  // k_ray work item: one block, 16 x 16 rays
-constexpr int NRAY = RTX * RTY;    // k_ray threads per block, one ray each
-constexpr int NBW = 8;             // march segments per ray per k_ray pass
 
 struct FilterDev {
   int kind, K, R;
@@ -81,10 +80,10 @@ struct BoneDev {
   float inv_scale[3], inv_trans[3];
   double pivot[12], pivot_inv[12], base[6];
   // per slot: the bone is scored in views view_of[0 .. n_slots), with that
-  // view's RayCaster settings and its empty-cell grid
+  // view's RayCaster settings and its clearance grid
   float step[MAX_SLOTS], scale[MAX_SLOTS];
   Cutoff cut[MAX_SLOTS];
-  const uint8_t* occ[MAX_SLOTS];
+  const uint8_t* clr[MAX_SLOTS];
   int view_of[MAX_SLOTS];
   int n_slots;
   int visible;                    // RayCaster::setVisible: a hidden volume renders zeros
@@ -107,16 +106,19 @@ struct IV {
   int rtx, rty, ftx, fty;
   int err;        // the crop exceeded the render size (the reference throws)
   float band[3];  // the bone's cutoff here: raw - t0, hi0 + t0, t1 (k_ray's band)
+  float step;     // the bone's sample distance here, and its volume's size (k_count_samples)
+  int nx, ny, nz;
   long long pix;  // offset of this crop in the DRR buffer
 };
 
 struct Counters {
   int n_items, n_iv;
   int rtiles, ftiles;
-  int rnext, fnext;
+  unsigned rnext;
+  int fnext;
   int error;
   int nfix;   // rays whose march met the cutoff's band (k_ray_fix marches them again)
-  int nfixt;  // ray tiles holding such rays
+  int nfixb;  // beams holding such rays
   int pad;
   unsigned long long samples, pixels;
   unsigned long long marched, slots;  // marched samples, 32 x warp-max span
@@ -134,7 +136,7 @@ struct Bufs {
   double* vcost;   // per iv
   unsigned* ivt;   // per-iv tile tickets
   unsigned* itt;   // per-item view tickets
-  int* fixt;       // ray tiles holding rays to march again exactly (k_ray_fix)
+  unsigned* fixb;  // beams (ray tile x BEAMS + its beam) holding rays to march again exactly (k_ray_fix)
   int* rtile_iv;   // per ray tile: its (item, view) (k_tile_map)
   int* ftile_iv;   // per view tile: its (item, view)
   Counters* C;
@@ -201,6 +203,10 @@ __device__ void setup_iv(const SceneDev* __restrict__ sc, int k, const int* __re
   r.band[0] = cut.raw - cut.t0;
   r.band[1] = cut.hi0 + cut.t0;
   r.band[2] = cut.t1;
+  r.step = B.step[j];
+  r.nx = B.vol.nx;
+  r.ny = B.vol.ny;
+  r.nz = B.vol.nz;
   double vc = 0.0;
   if (!calculate_viewport(mv, V.cam, V.ip, B.inv_scale, B.inv_trans, vp)) {
     vc = 9999.0;  // Tracker.cpp:614-617
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(1024) k_setup(const SceneDev* __restrict__ sc,
     b.C->fnext = 0;
     b.C->error = s_err;
     b.C->nfix = 0;
-    b.C->nfixt = 0;
+    b.C->nfixb = 0;
     b.C->samples = 0;
     b.C->marched = 0;
     b.C->slots = 0;
@@ -341,260 +347,104 @@ __global__ void __launch_bounds__(256) k_tile_map(Bufs b)
 #define ASC_RAY_MINBLOCKS 4  // 4 x 256 threads resident per SM (<= 64 registers)
 #endif
 
-// Rays of one 16 x 16 tile of one (item, view) crop per block.  Each ray's
-// march is cut into segments: the REBASE-sample march blocks that hold
-// occupied samples, each trimmed to its occupied extent (walk_segments).
-// The block's segments are sorted by length (counting sort, longest first)
-// and marched 32 at a time by whichever warp is free, so the lanes of a warp
-// march segments of nearly equal length whatever the rays' lengths; each ray
-// then adds its blocks' sums in order (add_block), as march() does for a
-// single ray.  A ray with more than NBW segments takes further passes.
-template <int STORE>
-__device__ __forceinline__ void march_segments(const DevVolume& V, const float4 (*rec)[NRAY], const unsigned* ord,
-                                               float* part, int nseg, int* grab, const float4* band,
-                                               const Cutoff& cut, unsigned long long& marched,
-                                               unsigned long long& slots)
+// The scene of one (item, view) record's rays.
+__device__ __forceinline__ RayScene ray_scene(const IV& r, const BoneDev& B, int skip)
 {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int g = 0;
-    if (lane == 0) g = atomicAdd(grab, 32);
-    g = __shfl_sync(FULL, g, 0);
-    if (g >= nseg) return;
-    int len = 0;
-    if (g + lane < nseg) {
-      const unsigned d = ord[g + lane];
-      const int slot = d & 2047u, js = (d >> 11) & 63u, je = (d >> 17) & 63u;
-      const int ray = slot / NBW;
-      RaySetup r;
-      const float4 q0 = rec[0][ray], q1 = rec[1][ray], q2 = rec[2][ray];
-      r.X = df{q0.x, q0.y};
-      r.Y = df{q0.z, q0.w};
-      r.Z = df{q1.x, q1.y};
-      r.dX = df{q1.z, q1.w};
-      r.dY = df{q2.x, q2.y};
-      r.dZ = df{q2.z, q2.w};
-      const int kb = __float_as_int(part[slot]);  // the block start, until the sum replaces it
-      // this ray's band: the tile's raw - t0, hi0 + t0 and t1 (cutoff_bounds)
-      const float4 c = *band;
-      const float S = fabsf(q1.z) + fabsf(q2.x) + fabsf(q2.z);
-      part[slot] = march_block<STORE, false>(V, r, kb, js, je, fmaf(-c.z, S, c.x), fmaf(c.z, S, c.y), cut);
-      len = je - js + 1;
-    }
-    const unsigned tot = __reduce_add_sync(FULL, (unsigned)len), mx = __reduce_max_sync(FULL, (unsigned)len);
-    marched += tot;
-    slots += 32ull * mx;
-  }
+  return RayScene{r.m, r.vp, df{r.sx[0], r.sx[1]}, df{r.sy[0], r.sy[1]}, B.step[r.slot],
+                  skip ? B.clr[r.slot] : nullptr, r.w, r.h};
 }
 
-// shape: log2 of the width of the ray block each warp takes in a 16 x 16
-// tile (2: 4 x 8, 3: 8 x 4, 4: 16 x 2), the autotuner's choice.  A ray any
-// of whose samples fell in the cutoff's band (march_block) leaves the mark
-// -1 in its DRR pixel, and its tile goes on the fix list for k_ray_fix.
+// The beams of the ray tiles, a warp each, from an atomic queue: a beam that
+// meets nothing (beam_mask) writes zeros, the others are marched (ray_beam).
+// shape: log2 of the width of a beam in its tile (2: 4 x 8 rays, 3: 8 x 4,
+// 4: 16 x 2), the autotuner's choice.  A ray any of whose samples fell in
+// the cutoff's band (march_block) leaves the mark -1 in its DRR pixel, and its
+// beam goes on the fix list for k_ray_fix.
 __global__ void __launch_bounds__(NRAY, ASC_RAY_MINBLOCKS) k_ray(const SceneDev* __restrict__ sc, Bufs b, int skip,
                                                                  int shape)
 {
-  static_assert(REBASE == 64 && NRAY * NBW <= 2048, "segment fields: 11-bit slot, 6-bit offsets");
-  __shared__ float4 s_rec[3][NRAY];      // per ray: X, Y, Z, dX, dY, dZ as double-floats
-  __shared__ float s_trim[3][NRAY];      // per ray: RayTrim's 1 / (8 dC) per axis (its C is in s_rec)
-  __shared__ float s_part[NRAY * NBW];   // per segment slot: the block start (int bits), then its sum
-  __shared__ unsigned s_seg[NRAY * NBW]; // per segment slot: slot | js << 11 | je << 17
-  __shared__ unsigned s_ord[NRAY * NBW]; // the segments, longest first
-  __shared__ int s_cnt[REBASE];          // segments per length - 1, then placement cursors
-  __shared__ int s_tile, s_nseg, s_grab, s_k;
-  __shared__ float4 s_band;              // the tile's cutoff: raw - t0, hi0 + t0, t1
-  __shared__ int s_fix;                  // 1 + the last tile, when one of its rays was marked
-  const unsigned FULL = 0xffffffffu;
-  const int tid = threadIdx.x, lane = tid & 31;
-  unsigned long long marched = 0, slots = 0, sampled = 0;
-  if (tid == 0) s_fix = 0;
+  __shared__ RaySlots S;
+  const int lane = threadIdx.x & 31;
+  const unsigned n = (unsigned)b.C->rtiles * BEAMS;
+  unsigned long long marched = 0, slots = 0;
+  unsigned next = 0;
+  if (lane == 0) next = atomicAdd(&b.C->rnext, 1u);
   for (;;) {
-    if (tid == 0) {
-      const int tl = atomicAdd(&b.C->rnext, 1);
-      s_tile = tl;
-      int kk = 0;
-      if (tl < b.C->rtiles) {
-        kk = b.rtile_iv[tl];
-        const float* bd = b.iv[kk].band;
-        s_band = make_float4(bd[0], bd[1], bd[2], 0.f);
-      }
-      s_k = kk;
-    }
-    __syncthreads();
-    // the last tile's mark (set after its last barrier, visible past this one)
-    if (tid == 0 && s_fix) {
-      b.fixt[atomicAdd(&b.C->nfixt, 1)] = s_fix - 1;
-      s_fix = 0;
-    }
-    const int tile = s_tile;
-    if (tile >= b.C->rtiles) break;
-    const int k = s_k;
+    const unsigned id = __shfl_sync(FULL_WARP, next, 0);
+    if (id >= n) break;
+    if (lane == 0) next = atomicAdd(&b.C->rnext, 1u);  // taken while this beam is marched
+    const int tile = (int)(id / BEAMS), k = b.rtile_iv[tile], t = tile - b.roff[k];
     const IV& r = b.iv[k];
-    const int t = tile - b.roff[k];
-    // each warp takes a (1 << shape) x (32 >> shape) block of the 16 x 16
-    // tile (coherent walks)
-    const int wsh = shape, wpr = 4 - shape;  // log2 of the block width, of the blocks per tile row
-    const int wrp = tid >> 5;
-    const int x = (t % r.rtx) * RTX + ((wrp & ((1 << wpr) - 1)) << wsh) + (lane & ((1 << wsh) - 1)),
-              y = (t / r.rtx) * RTY + ((wrp >> wpr) << (5 - wsh)) + (lane >> wsh);
+    int x, y;
+    beam_pixel((t % r.rtx) * RTX, (t / r.rtx) * RTY, (int)(id % BEAMS), shape, x, y);
     const bool valid = x < r.w && y < r.h;
+    if (!__any_sync(FULL_WARP, valid)) continue;
     const BoneDev& B = sc->bones[r.bone];
-    const int j = r.slot;
-    const Cutoff& cut = B.cut[j];
-    const uint8_t* occ = skip ? B.occ[j] : nullptr;
-    RaySetup rs{};
-    const bool hit = valid && ray_setup(r.m, r.vp, x, y, df{r.sx[0], r.sx[1]}, df{r.sy[0], r.sy[1]}, B.step[j],
-                                        B.vol.nx, B.vol.ny, B.vol.nz, rs);
-    // trilinear samples of the reference's march (the work figure of the
-    // roofline), counted per warp and added to the global count once at the end
-    sampled += __reduce_add_sync(FULL, hit ? (unsigned)rs.K : 0u);
-    bool done = true;
-    CellWalk cw = cell_walk(B.vol, rs, 0);
-    if (hit && rs.K > 0) {
-      s_rec[0][tid] = make_float4(rs.X.h, rs.X.l, rs.Y.h, rs.Y.l);
-      s_rec[1][tid] = make_float4(rs.Z.h, rs.Z.l, rs.dX.h, rs.dX.l);
-      s_rec[2][tid] = make_float4(rs.dY.h, rs.dY.l, rs.dZ.h, rs.dZ.l);
-      // ray_trim's 1 / (8 dC) from the walk's crossing intervals (dt = 8 / |dC|)
-      const bool big = B.vol.nx > OCC_TRIM_MAX || B.vol.ny > OCC_TRIM_MAX || B.vol.nz > OCC_TRIM_MAX;
-      const float nan = __int_as_float(0x7fffffff);
-      s_trim[0][tid] = big || cw.ix == 0 ? nan : (cw.ix < 0 ? cw.dtx : -cw.dtx) * (1.0f / 64.0f);
-      s_trim[1][tid] = big || cw.iy == 0 ? nan : (cw.iy < 0 ? cw.dty : -cw.dty) * (1.0f / 64.0f);
-      s_trim[2][tid] = big || cw.iz == 0 ? nan : (cw.iz < 0 ? cw.dtz : -cw.dtz) * (1.0f / 64.0f);
-      done = false;
+    const RayScene s = ray_scene(r, B, skip);
+    const Beam beam = beam_mask(B.vol, s, min(x, r.w - 1), min(y, r.h - 1));
+    float* out = b.drr + r.pix + (long long)y * r.w + x;
+    if (!beam.mask) {
+      if (valid) *out = 0.f;
+      continue;
     }
-    WalkState ws{0, rs.K - 1, 0, -1, 0};
-    df total{0.f, 0.f};  // NaN once a segment met the cutoff's band
-    for (;;) {
-      if (tid < REBASE) s_cnt[tid] = 0;
-      if (tid == 0) s_grab = 0;
-      __syncthreads();
-      // ---- walk: up to NBW segments of this ray
-      int n = 0;
-      const auto trim = [&](int i, float& ia, float& c) {
-        ia = s_trim[i][tid];
-        c = i == 0 ? s_rec[0][tid].x : (i == 1 ? s_rec[0][tid].z : s_rec[1][tid].x);  // X.h, Y.h, Z.h
-      };
-      if (!done)
-        done = walk_segments(cw, occ, trim, ws, [&](int kb, int js, int je) {
-          if (n == NBW) return false;
-          const int slot = tid * NBW + n++;
-          s_seg[slot] = (unsigned)slot | (unsigned)js << 11 | (unsigned)je << 17;
-          s_part[slot] = __int_as_float(kb);
-          atomicAdd(&s_cnt[je - js], 1);
-          return true;
-        });
-      __syncthreads();
-      // ---- counting sort by length, longest first
-      if (tid < 32) {
-        const int c0 = s_cnt[REBASE - 1 - 2 * lane], c1 = s_cnt[REBASE - 2 - 2 * lane];
-        int incl = c0 + c1;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(FULL, incl, o);
-          if (lane >= o) incl += u;
-        }
-        const int excl = incl - c0 - c1;
-        s_cnt[REBASE - 1 - 2 * lane] = excl;
-        s_cnt[REBASE - 2 - 2 * lane] = excl + c0;
-        if (lane == 31) s_nseg = incl;
-      }
-      __syncthreads();
-      for (int i = 0; i < n; ++i) {
-        const unsigned d = s_seg[tid * NBW + i];
-        const int len1 = (int)((d >> 17) & 63u) - (int)((d >> 11) & 63u);
-        s_ord[atomicAdd(&s_cnt[len1], 1)] = d;
-      }
-      __syncthreads();
-      const int nseg = s_nseg;
-      // ---- march the segments, 32 at a time per warp
-      if (B.vol.storage == ASC_STORE_F32)
-        march_segments<ASC_STORE_F32>(B.vol, s_rec, s_ord, s_part, nseg, &s_grab, &s_band, cut, marched,
-                                      slots);
-      else if (B.vol.storage == ASC_STORE_BF16)
-        march_segments<ASC_STORE_BF16>(B.vol, s_rec, s_ord, s_part, nseg, &s_grab, &s_band, cut, marched,
-                                      slots);
-      else if (B.vol.storage == ASC_STORE_F16)
-        march_segments<ASC_STORE_F16>(B.vol, s_rec, s_ord, s_part, nseg, &s_grab, &s_band, cut, marched,
-                                      slots);
-      else
-        march_segments<ASC_STORE_U16>(B.vol, s_rec, s_ord, s_part, nseg, &s_grab, &s_band, cut, marched,
-                                      slots);
-      __syncthreads();
-      // ---- this ray's segments, in order
-      for (int i = 0; i < n; ++i) {
-        const float p = s_part[tid * NBW + i];
-        if (block_flagged(p))
-          total.h = __int_as_float(0x7fffffff);  // NaN stays NaN through add_block
-        else
-          add_block(total, p);
-      }
-      if (!__syncthreads_or(!done)) break;
-    }
-    if (valid) {
-      const bool flagged = total.h != total.h;
-      b.drr[r.pix + (long long)y * r.w + x] =
-          flagged ? -1.0f : fminf(fmaxf((total.h + total.l) * B.scale[j], 0.f), 1.f);
-      if (flagged) s_fix = tile + 1;
-    }
+    unsigned done = 0, room = 0;
+    const float d = ray_beam(B.vol, s, B.cut[r.slot], make_float4(r.band[0], r.band[1], r.band[2], 0.f), S, x, y, valid,
+                             beam, done, room);
+    marched += done;
+    slots += room;
+    const bool flagged = valid && d != d;
+    if (valid) *out = flagged ? -1.0f : fminf(fmaxf(d * B.scale[r.slot], 0.f), 1.f);
+    if (__any_sync(FULL_WARP, flagged) && lane == 0) b.fixb[atomicAdd(&b.C->nfixb, 1)] = id;
   }
-  if (lane == 0 && sampled) atomicAdd(&b.C->samples, sampled);
   if (lane == 0 && slots) {
     atomicAdd(&b.C->marched, marched);
     atomicAdd(&b.C->slots, slots);
   }
 }
 
-// The marked rays of the tiles on the fix list, marched again with every
-// cutoff decision the exact one (march_pass with EXACT); each overwrites its
-// mark.  A warp per listed tile: its marked rays, found by ballots over the
-// tile's 256 pixels, are dealt to the lanes, so a tile's rays march side by
-// side.  The ray set-up is k_ray's, so the samples are the same.
+// The marked rays of the beams on the fix list, marched again with every
+// cutoff decision the exact one; each overwrites its mark.  Each takes a
+// whole warp (march_exact), one after the other within a beam.
 constexpr int FIX_THREADS = 128;
-__global__ void __launch_bounds__(FIX_THREADS) k_ray_fix(const SceneDev* __restrict__ sc, Bufs b, int skip)
+__global__ void __launch_bounds__(FIX_THREADS) k_ray_fix(const SceneDev* __restrict__ sc, Bufs b, int shape)
 {
-  __shared__ unsigned char s_pix[FIX_THREADS / 32][NRAY];  // per warp: the tile's marked rays
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nt = b.C->nfixt;
+  __shared__ float s_v[FIX_THREADS / 32][EXACT_FLOATS];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n = b.C->nfixb;
   const int nw = gridDim.x * (FIX_THREADS / 32);
-  for (int w = blockIdx.x * (FIX_THREADS / 32) + wib; w < nt; w += nw) {
-    const int tile = b.fixt[w];
-    const int k = b.rtile_iv[tile];
+  for (int i = wib * gridDim.x + blockIdx.x; i < n; i += nw) {
+    const unsigned id = b.fixb[i];
+    const int tile = (int)(id / BEAMS), k = b.rtile_iv[tile], t = tile - b.roff[k];
     const IV& r = b.iv[k];
-    const int t = tile - b.roff[k];
-    const int x0 = (t % r.rtx) * RTX, y0 = (t / r.rtx) * RTY;
-    int cnt = 0;
-    for (int c = 0; c < NRAY / 32; ++c) {
-      const int p = c * 32 + lane, x = x0 + p % RTX, y = y0 + p / RTX;
-      const bool marked = x < r.w && y < r.h && b.drr[r.pix + (long long)y * r.w + x] < 0.f;
-      const unsigned m = __ballot_sync(0xffffffffu, marked);
-      if (marked) s_pix[wib][cnt + __popc(m & ((1u << lane) - 1u))] = (unsigned char)p;
-      cnt += __popc(m);
-    }
-    __syncwarp();
-    if (lane == 0) atomicAdd(&b.C->nfix, cnt);
+    int x, y;
+    beam_pixel((t % r.rtx) * RTX, (t / r.rtx) * RTY, (int)(id % BEAMS), shape, x, y);
     const BoneDev& B = sc->bones[r.bone];
-    const int j = r.slot;
-    const uint8_t* occ = skip ? B.occ[j] : nullptr;
-    for (int i = lane; i < cnt; i += 32) {
-      const int p = s_pix[wib][i], x = x0 + p % RTX, y = y0 + p / RTX;
-      RaySetup rs;
-      float d = 0.f;
-      if (ray_setup(r.m, r.vp, x, y, df{r.sx[0], r.sx[1]}, df{r.sy[0], r.sy[1]}, B.step[j], B.vol.nx, B.vol.ny,
-                    B.vol.nz, rs) &&
-          rs.K > 0) {
-        if (B.vol.storage == ASC_STORE_F32)
-          d = march_pass<ASC_STORE_F32, true>(B.vol, occ, rs, B.cut[j], nullptr);
-        else if (B.vol.storage == ASC_STORE_BF16)
-          d = march_pass<ASC_STORE_BF16, true>(B.vol, occ, rs, B.cut[j], nullptr);
-        else if (B.vol.storage == ASC_STORE_F16)
-          d = march_pass<ASC_STORE_F16, true>(B.vol, occ, rs, B.cut[j], nullptr);
-        else
-          d = march_pass<ASC_STORE_U16, true>(B.vol, occ, rs, B.cut[j], nullptr);
-      }
-      b.drr[r.pix + (long long)y * r.w + x] = fminf(fmaxf(d * B.scale[j], 0.f), 1.f);
+    const RayScene s = ray_scene(r, B, 0);
+    unsigned m = __ballot_sync(FULL_WARP, x < r.w && y < r.h && b.drr[r.pix + (long long)y * r.w + x] < 0.f);
+    if (lane == 0) atomicAdd(&b.C->nfix, __popc(m));
+    for (; m; m &= m - 1) {
+      const int rx = __shfl_sync(FULL_WARP, x, __ffs(m) - 1), ry = __shfl_sync(FULL_WARP, y, __ffs(m) - 1);
+      const float d = march_exact(B.vol, s, B.cut[r.slot], rx, ry, s_v[wib]);
+      if (lane == 0) b.drr[r.pix + (long long)ry * r.w + rx] = fminf(fmaxf(d * B.scale[r.slot], 0.f), 1.f);
     }
-    __syncwarp();
   }
+}
+
+// Trilinear samples of the reference's march over the last evaluation's
+// crops, from their records (asc_engine_stats, asc_engine_counters): the
+// evaluation itself sets up only the rays that meet an occupied interval.
+__global__ void __launch_bounds__(NRAY) k_count_samples(Bufs b)
+{
+  unsigned long long n = 0;
+  for (int tile = blockIdx.x; tile < b.C->rtiles; tile += gridDim.x) {
+    const int k = b.rtile_iv[tile], t = tile - b.roff[k];
+    const IV& r = b.iv[k];
+    const int x = (t % r.rtx) * RTX + threadIdx.x % RTX, y = (t / r.rtx) * RTY + threadIdx.x / RTX;
+    RaySetup rs;
+    const bool hit = x < r.w && y < r.h && ray_setup(r.m, r.vp, x, y, df{r.sx[0], r.sx[1]}, df{r.sy[0], r.sy[1]},
+                                                     r.step, r.nx, r.ny, r.nz, rs);
+    n += __reduce_add_sync(FULL_WARP, hit ? (unsigned)rs.K : 0u);
+  }
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(&b.C->samples, n);
 }
 
 // ---------------------------------------------------------------- k_view
@@ -1317,14 +1167,14 @@ struct asc_engine_s {
   float *p_drr = nullptr, *p_rad = nullptr, *p_mask = nullptr, *p_bg = nullptr, *p_tmp = nullptr, *p_bgr = nullptr;
   double* p_res = nullptr;
   std::vector<void*> allocs;
-  // empty-cell grids of bones replaced by asc_engine_set_bone, per (bone,
+  // clearance grids of bones replaced by asc_engine_set_bone, per (bone,
   // slot), with their capacity in bytes
-  uint8_t* occ_own[MAX_BONES][MAX_SLOTS] = {};
-  size_t occ_cap[MAX_BONES][MAX_SLOTS] = {};
+  uint8_t* clr_own[MAX_BONES][MAX_SLOTS] = {};
+  size_t clr_cap[MAX_BONES][MAX_SLOTS] = {};
   ~asc_engine_s()
   {
     for (void* p : allocs) cudaFree(p);
-    for (auto& row : occ_own)
+    for (auto& row : clr_own)
       for (uint8_t* p : row)
         if (p) cudaFree(p);
     for (cudaEvent_t x : ev)
@@ -1491,13 +1341,17 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
       B.step[j] = bones[i].step[j];
       B.scale[j] = bones[i].step[j] * vh->dev.norm / bones[i].intensity[j];
       B.cut[j] = make_cutoff(bones[i].cutoff[j], vh->dev.norm, vh->dev.gmax);
-      uint8_t* occ = nullptr;
-      if (e->alloc(occ, occ_grid_bytes(occupancy_cells(vh->dev)))) {
+      uint8_t* clr = nullptr;
+      if (e->alloc(clr, clearance_cells(vh->dev))) {
         delete e;
         return ASC_ERR_NOMEM;
       }
-      build_occupancy(vh->dev, occupancy_threshold(B.cut[j]), occ, cs);
-      B.occ[j] = occ;
+      int rc = build_clearance(vh->dev, occupancy_threshold(B.cut[j]), clr, cs);
+      if (rc) {
+        delete e;
+        return rc;
+      }
+      B.clr[j] = clr;
     }
   }
   e->max_items = max_items;
@@ -1519,8 +1373,9 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
   if (!err) err = e->alloc(e->b.ivt, n_iv);
   if (!err) err = e->alloc(e->b.itt, (size_t)max_items);
   // at most every ray tile of a full batch
-  if (!err) err = e->alloc(e->b.fixt, n_iv * (size_t)((rw + RTX - 1) / RTX) * ((rh + RTY - 1) / RTY));
-  if (!err) err = e->alloc(e->b.rtile_iv, n_iv * (size_t)((rw + RTX - 1) / RTX) * ((rh + RTY - 1) / RTY));
+  const size_t ray_tiles = n_iv * (size_t)((rw + RTX - 1) / RTX) * ((rh + RTY - 1) / RTY);
+  if (!err) err = e->alloc(e->b.fixb, ray_tiles * BEAMS);
+  if (!err) err = e->alloc(e->b.rtile_iv, ray_tiles);
   if (!err) err = e->alloc(e->b.C, 1);
   if (!err) err = e->alloc(e->d_bone, (size_t)max_items);
   if (!err) err = e->alloc(e->d_manip, (size_t)max_items * 6);
@@ -1656,22 +1511,23 @@ ASC_API int asc_engine_set_bone(asc_engine e, int bone, const asc_bone_desc* des
   B.visible = 1;
   B.n_slots = n_views;
   Gate g(device_gate());
-  const size_t grid = occ_grid_bytes(occupancy_cells(vh->dev));
+  const size_t grid = clearance_cells(vh->dev);
   for (int j = 0; j < n_views; ++j) {
     B.view_of[j] = views[j];
     B.step[j] = desc->step[j];
     B.scale[j] = desc->step[j] * vh->dev.norm / desc->intensity[j];
     B.cut[j] = make_cutoff(desc->cutoff[j], vh->dev.norm, vh->dev.gmax);
-    uint8_t*& occ = e->occ_own[bone][j];
-    if (e->occ_cap[bone][j] < grid) {
-      if (occ) cudaFree(occ);
-      occ = nullptr;
-      e->occ_cap[bone][j] = 0;
-      ASC_CUDA(cudaMalloc(&occ, grid));
-      e->occ_cap[bone][j] = grid;
+    uint8_t*& clr = e->clr_own[bone][j];
+    if (e->clr_cap[bone][j] < grid) {
+      if (clr) cudaFree(clr);
+      clr = nullptr;
+      e->clr_cap[bone][j] = 0;
+      ASC_CUDA(cudaMalloc(&clr, grid));
+      e->clr_cap[bone][j] = grid;
     }
-    build_occupancy(vh->dev, occupancy_threshold(B.cut[j]), occ, nullptr);
-    B.occ[j] = occ;
+    int rc = build_clearance(vh->dev, occupancy_threshold(B.cut[j]), clr, nullptr);
+    if (rc) return rc;
+    B.clr[j] = clr;
   }
   ASC_CUDA(cudaStreamSynchronize(nullptr));
   e->host.bones[bone] = B;
@@ -1798,7 +1654,7 @@ static int engine_launch(asc_engine e, int n, const int* bone, const double* man
   k_tile_map<<<e->sms * 2, 256, 0, s>>>(e->b);
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[1], s));
   k_ray<<<e->sms * e->launch.ray_blocks_per_sm, NRAY, 0, s>>>(e->dev, e->b, g_empty_skip, e->launch.ray_shape);
-  k_ray_fix<<<e->sms * 4, FIX_THREADS, 0, s>>>(e->dev, e->b, g_empty_skip);
+  k_ray_fix<<<e->sms * 4, FIX_THREADS, 0, s>>>(e->dev, e->b, e->launch.ray_shape);
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[2], s));
   k_view<<<e->sms * e->view_grid(), VNT, e->smem, s>>>(e->dev, e->b, cost, vcost);
   if (e->host.cf_model) k_sad<<<e->sms * 8, 256, 0, s>>>(e->dev, e->b, cost, vcost);
@@ -1817,6 +1673,16 @@ ASC_API int asc_engine_profile(asc_engine e, int enable)
   return ASC_OK;
 }
 
+// The last evaluation's counters, its samples counted here.
+static int read_counters(asc_engine e, Counters& C)
+{
+  ASC_CUDA(cudaMemset(&e->b.C->samples, 0, sizeof C.samples));
+  k_count_samples<<<e->sms * 8, NRAY>>>(e->b);
+  ASC_LAUNCH_CHECK();
+  ASC_CUDA(cudaMemcpy(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost));
+  return ASC_OK;
+}
+
 ASC_API int asc_engine_stats(asc_engine e, float ms[3], unsigned long long* samples, unsigned long long* pixels)
 {
   if (!e) return ASC_ERR_ARG;
@@ -1826,7 +1692,8 @@ ASC_API int asc_engine_stats(asc_engine e, float ms[3], unsigned long long* samp
     for (int i = 0; i < 3; ++i) ASC_CUDA(cudaEventElapsedTime(&ms[i], e->ev[i], e->ev[i + 1]));
   }
   Counters C;
-  ASC_CUDA(cudaMemcpy(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost));
+  int rc = read_counters(e, C);
+  if (rc) return rc;
   if (samples) *samples = C.samples;
   if (pixels) *pixels = C.pixels;
   return ASC_OK;
@@ -1845,7 +1712,8 @@ ASC_API int asc_engine_counters(asc_engine e, unsigned long long out[4])
 {
   if (!e || !out) return ASC_ERR_ARG;
   Counters C;
-  ASC_CUDA(cudaMemcpy(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost));
+  int rc = read_counters(e, C);
+  if (rc) return rc;
   out[0] = C.samples;
   out[1] = C.pixels;
   out[2] = C.marched;
@@ -2047,7 +1915,7 @@ static int render_bone(const BoneDev& B, const asc_bone_desc& BD, int v, const f
     ASC_CUDA(cudaMemsetAsync(out, 0, (size_t)w * h * sizeof(float), s));
     return ASC_OK;
   }
-  return raycast_launch(B.vol, g_empty_skip ? B.occ[v] : nullptr, m, vpf, BD.step[v], BD.intensity[v], BD.cutoff[v],
+  return raycast_launch(B.vol, g_empty_skip ? B.clr[v] : nullptr, m, vpf, BD.step[v], BD.intensity[v], BD.cutoff[v],
                         out, w, h, s);
 }
 
@@ -2384,7 +2252,7 @@ ASC_API int asc_engine_render_drr(asc_engine e, int view, const double* poses, c
     float m[12];
     view_matrix(V, B, poses + 6 * b, m);
     if (!B.visible) continue;  // its zeros leave the merge unchanged
-    int rc = raycast_launch(B.vol, g_empty_skip ? B.occ[view] : nullptr, m, vpf, BD.step[view], BD.intensity[view],
+    int rc = raycast_launch(B.vol, g_empty_skip ? B.clr[view] : nullptr, m, vpf, BD.step[view], BD.intensity[view],
                             BD.cutoff[view], e->p_drr, w, h, s);
     if (!rc) rc = asc_merge(e->p_mask, e->p_drr, e->p_mask, w, h, s);
     if (rc) return rc;

@@ -47,8 +47,8 @@ namespace asc {
 struct asc_volume_host {
   DevVolume dev;
   uint32_t* pairs;
-  uint8_t* occ;     // occupancy grid of the plain ray caster ...
-  float occ_cutoff; // ... for this raw cutoff (NaN = not built)
+  uint8_t* clr;     // clearance grid of the plain ray caster ...
+  float clr_cutoff; // ... for this raw cutoff (NaN = not built)
   float inv_scale[3], inv_trans[3];
   double trans_center[3];
   float min_value, max_value;
@@ -56,11 +56,12 @@ struct asc_volume_host {
   int bps;
 };
 
-// Builds the occupancy grid of a device volume for one raw cutoff.
-void build_occupancy(const DevVolume& V, float cutoff_raw, uint8_t* occ, cudaStream_t s);
-inline size_t occupancy_cells(const DevVolume& V)
+// Builds the clearance grid (a byte per cell) of a device volume for one raw
+// cutoff.
+int build_clearance(const DevVolume& V, float cutoff_raw, uint8_t* clr, cudaStream_t s);
+inline size_t clearance_cells(const DevVolume& V)
 {
-  return (size_t)occ_dim(V.nx) * occ_dim(V.ny) * occ_dim(V.nz);
+  return (size_t)clear_dim(V.nx) * clear_dim(V.ny) * clear_dim(V.nz);
 }
 
 // Global switches (asc_set_option).
@@ -523,7 +524,7 @@ int gauss_1d(float radius, float* g, int cap);
 int launch_filter(const asc_filter_desc& f, const float* in, float* out, int w, int h, cudaStream_t s);
 
 // One plain ray-cast launch with an already folded float matrix.
-int raycast_launch(const DevVolume& V, const uint8_t* occ, const float* m12, const float* vp, float step,
+int raycast_launch(const DevVolume& V, const uint8_t* clr, const float* m12, const float* vp, float step,
                    float intensity, float cutoff, float* out, int w, int h, cudaStream_t s);
 
 }  // namespace asc

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "asc_internal.cuh"
+#include "asc_rays.cuh"
 
 namespace asc {
 
@@ -47,9 +48,9 @@ int gauss_1d(float radius, float* g, int cap)
 
 // ---------------------------------------------------------------- kernels
 
-// cuda_volume_render_kernel (RayCaster_kernels.cu:144-195) for one image.
-// 16x16 pixel blocks; each warp covers an 8x4 sub-tile so that its rays
-// sample neighbouring voxels.
+// cuda_volume_render_kernel (RayCaster_kernels.cu:144-195) for one image: a
+// warp per beam of 8 x 4 pixels (ray_beam).  Rays with a sample in the
+// cutoff's band are marched again, exactly, by their warp.
 struct RayArgs {
   float m[12];
   float vp[4];
@@ -58,19 +59,31 @@ struct RayArgs {
   float sx[2], sy[2];  // vp[2] / w and vp[3] / h as double-floats
 };
 
-template <int STORE>
-__global__ void __launch_bounds__(256) k_raycast(DevVolume V, const uint8_t* __restrict__ occ, RayArgs a,
-                                                 float* __restrict__ out, int w, int h)
+__global__ void __launch_bounds__(NRAY, 4) k_raycast(DevVolume V, const uint8_t* __restrict__ clr,
+                                                     const __grid_constant__ RayArgs a, float* __restrict__ out, int w,
+                                                     int h)
 {
+  __shared__ RaySlots S;
+  __shared__ float s_v[NRAY / 32][EXACT_FLOATS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-  const int y = blockIdx.y * 16 + (warp >> 1) * 4 + (lane >> 3);
-  if (x >= w || y >= h) return;
-  RaySetup r;
+  int x, y;
+  beam_pixel(blockIdx.x * RTX, blockIdx.y * RTY, warp, 3, x, y);
+  const bool valid = x < w && y < h;
+  const RayScene s{a.m, a.vp, df{a.sx[0], a.sx[1]}, df{a.sy[0], a.sy[1]}, a.step, clr, w, h};
+  const Beam b = beam_mask(V, s, min(x, w - 1), min(y, h - 1));
   float d = 0.f;
-  if (ray_setup(a.m, a.vp, x, y, df{a.sx[0], a.sx[1]}, df{a.sy[0], a.sy[1]}, a.step, V.nx, V.ny, V.nz, r))
-    d = march<STORE>(V, occ, r, a.cut) * a.scale;
-  out[(size_t)y * w + x] = fminf(fmaxf(d, 0.f), 1.f);
+  if (b.mask) {
+    unsigned marched = 0, slots = 0;
+    d = ray_beam(V, s, a.cut, make_float4(a.cut.raw - a.cut.t0, a.cut.hi0 + a.cut.t0, a.cut.t1, 0.f), S, x, y, valid, b,
+                 marched, slots);
+    for (unsigned m = __ballot_sync(FULL_WARP, valid && d != d); m; m &= m - 1) {
+      const int q = __ffs(m) - 1;
+      const int rx = __shfl_sync(FULL_WARP, x, q), ry = __shfl_sync(FULL_WARP, y, q);
+      const float e = march_exact(V, s, a.cut, rx, ry, s_v[warp]);
+      if (lane == q) d = e;
+    }
+  }
+  if (valid) out[(size_t)y * w + x] = fminf(fmaxf(d * a.scale, 0.f), 1.f);
 }
 
 // image_render_kernel (RadRenderer_kernels.cu:85-116) and
@@ -409,39 +422,91 @@ __global__ void __launch_bounds__(RB) k_hdist_sad(const float* __restrict__ f, c
   }
 }
 
-// Occupancy bytes and boxes of OCC^3-voxel cells (occ_cell in asc_march.cuh),
-// margin cells included: one thread per cell scans the cell and its apron
-// (voxels outside the volume are 0).
-template <int STORE>
-__global__ void k_occupancy(DevVolume V, float cutoff_raw, uint8_t* __restrict__ occ)
+// The clearance grid (asc_march.cuh) of CB^3 cells per block.  The maximum
+// norm is separable, so the distance is taken along x, then y, then z, in
+// shared memory: a 64-bit word per row of the block's voxels and CLEAR_MAX
+// around them, a byte per (cell x, y, z), a byte per (cell x, cell y, z), and
+// the cells.  Every voxel is read (62 / 32)^3 = 7 times, from L2.
+constexpr int CB = 16;                              // cells of a block's edge
+constexpr int CV = CLEAR_CELL * CB + 2 * CLEAR_MAX;  // voxels of its edge, the surroundings included
+constexpr int CLEAR_THREADS = 512;
+constexpr size_t CLEAR_SMEM = (size_t)CV * CV * 8 + (size_t)CB * CV * CV + (size_t)CB * CB * CV;
+static_assert(CV <= 64, "a row of voxels is a 64-bit word");
+
+// min over the cell's surroundings of max(distance along the axis, d[i *
+// stride]): cell c covers entries [CLEAR_MAX + 2c, CLEAR_MAX + 2c + 2], those at distance 0.
+__device__ __forceinline__ int clear_along(const uint8_t* d, int stride, int c)
 {
-  const int px = occ_dim(V.nx), py = occ_dim(V.ny), pz = occ_dim(V.nz);
-  const int n = px * py * pz;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  const int cx = c % px - OCC_PAD, cy = (c / px) % py - OCC_PAD, cz = c / (px * py) - OCC_PAD;
-  int box[4];
-  occ[c] = occ_cell(cx, cy, cz, V.nx, V.ny, V.nz, cutoff_raw,
-                    [&](int x, int y, int z) {
-                      return voxel_value<STORE>(V, (size_t)(z + PAD) * V.pxy + (size_t)(y + PAD) * V.px + (x + PAD));
-                    },
-                    box);
-  reinterpret_cast<int4*>(occ + occ_box_offset((size_t)n))[c] = make_int4(box[0], box[1], box[2], box[3]);
+  const uint8_t* p = d + (CLEAR_MAX + CLEAR_CELL * c) * stride;
+  int e = min((int)p[0], min((int)p[stride], (int)p[2 * stride]));
+  for (int i = 1; i < CLEAR_MAX && i < e; ++i) {
+    e = min(e, max(i, (int)p[-i * stride]));
+    if (CLEAR_MAX + CLEAR_CELL * c + CLEAR_CELL + i < CV) e = min(e, max(i, (int)p[(CLEAR_CELL + i) * stride]));
+  }
+  return e;
+}
+
+template <int STORE>
+__global__ void __launch_bounds__(CLEAR_THREADS) k_clearance(DevVolume V, float cutoff_raw, uint8_t* __restrict__ clr)
+{
+  extern __shared__ unsigned long long clear_sm[];
+  unsigned long long* rows = clear_sm;               // [z][y]
+  uint8_t* dx = (uint8_t*)(rows + CV * CV);          // [z][y][cell x]
+  uint8_t* dy = dx + CB * CV * CV;                   // [z][cell y][cell x]
+  const int gx = clear_dim(V.nx), gy = clear_dim(V.ny), gz = clear_dim(V.nz);
+  const int cx0 = blockIdx.x * CB, cy0 = blockIdx.y * CB, cz0 = blockIdx.z * CB;
+  const int x0 = CLEAR_CELL * cx0 - CLEAR_MAX, y0 = CLEAR_CELL * cy0 - CLEAR_MAX, z0 = CLEAR_CELL * cz0 - CLEAR_MAX;
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i < CV * CV; i += CLEAR_THREADS / 32) {  // a warp per row
+    const int y = y0 + i % CV, z = z0 + i / CV;
+    unsigned long long bits = 0;
+    if (y >= 0 && y < V.ny && z >= 0 && z < V.nz)
+      for (int half = 0; half < 2; ++half) {
+        const int x = x0 + 32 * half + lane;
+        const bool above = x >= 0 && x < V.nx && 32 * half + lane < CV &&
+                           voxel_value<STORE>(V, (size_t)(z + PAD) * V.pxy + (size_t)(y + PAD) * V.px + (x + PAD)) > cutoff_raw;
+        bits |= (unsigned long long)__ballot_sync(FULL_WARP, above) << (32 * half);
+      }
+    if (lane == 0) rows[i] = bits;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < CB * CV * CV; i += CLEAR_THREADS) {
+    // the row's voxels from 2c - 15 on: bits 15 .. 17 are at distance 0, bit
+    // 14 - d lies d + 1 before the cell, bit 17 + d d past it
+    const unsigned long long m = rows[i / CB] >> (CLEAR_CELL * (i % CB));
+    const unsigned before = (unsigned)m & ((1u << CLEAR_MAX) - 1u);
+    const unsigned past = (unsigned)(m >> CLEAR_MAX) & ((1u << (CLEAR_MAX + CLEAR_CELL)) - 1u);
+    int e = CLEAR_MAX;
+    if (before) e = min(e, CLEAR_MAX - (31 - __clz(before)));
+    if (past) e = min(e, max(0, __ffs(past) - 1 - CLEAR_CELL));
+    dx[i] = (uint8_t)e;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < CB * CB * CV; i += CLEAR_THREADS) {
+    const int cx = i % CB, cy = i / CB % CB, z = i / (CB * CB);
+    dy[i] = (uint8_t)clear_along(dx + z * CV * CB + cx, CB, cy);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < CB * CB * CB; i += CLEAR_THREADS) {
+    const int cx = i % CB, cy = i / CB % CB, cz = i / (CB * CB);
+    if (cx0 + cx < gx && cy0 + cy < gy && cz0 + cz < gz)
+      clr[((size_t)(cz0 + cz) * gy + (cy0 + cy)) * gx + (cx0 + cx)] = (uint8_t)clear_along(dy + cy * CB + cx, CB * CB, cz);
+  }
 }
 
 int g_empty_skip = 1;
 
-void build_occupancy(const DevVolume& V, float cutoff_raw, uint8_t* occ, cudaStream_t s)
+int build_clearance(const DevVolume& V, float cutoff_raw, uint8_t* clr, cudaStream_t s)
 {
-  int n = (int)occupancy_cells(V);
-  if (V.storage == ASC_STORE_F32)
-    k_occupancy<ASC_STORE_F32><<<(n + 127) / 128, 128, 0, s>>>(V, cutoff_raw, occ);
-  else if (V.storage == ASC_STORE_BF16)
-    k_occupancy<ASC_STORE_BF16><<<(n + 127) / 128, 128, 0, s>>>(V, cutoff_raw, occ);
-  else if (V.storage == ASC_STORE_F16)
-    k_occupancy<ASC_STORE_F16><<<(n + 127) / 128, 128, 0, s>>>(V, cutoff_raw, occ);
-  else
-    k_occupancy<ASC_STORE_U16><<<(n + 127) / 128, 128, 0, s>>>(V, cutoff_raw, occ);
+  const auto kernel = V.storage == ASC_STORE_F32    ? k_clearance<ASC_STORE_F32>
+                      : V.storage == ASC_STORE_BF16 ? k_clearance<ASC_STORE_BF16>
+                      : V.storage == ASC_STORE_F16  ? k_clearance<ASC_STORE_F16>
+                                                    : k_clearance<ASC_STORE_U16>;
+  ASC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLEAR_SMEM));
+  const dim3 grid((clear_dim(V.nx) + CB - 1) / CB, (clear_dim(V.ny) + CB - 1) / CB, (clear_dim(V.nz) + CB - 1) / CB);
+  kernel<<<grid, CLEAR_THREADS, CLEAR_SMEM, s>>>(V, cutoff_raw, clr);
+  ASC_LAUNCH_CHECK();
+  return ASC_OK;
 }
 
 // ---------------------------------------------------------------- host side
@@ -759,8 +824,8 @@ ASC_API int asc_volume_create(const void* data, int W, int H, int D, int bps, co
       2147483648.0)
     return ASC_ERR_RANGE;
   auto* v = new asc_volume_host();
-  v->occ = nullptr;
-  v->occ_cutoff = NAN;
+  v->clr = nullptr;
+  v->clr_cutoff = NAN;
   int dims[3] = {mx[0] - mn[0] + 1, mx[1] - mn[1] + 1, mx[2] - mn[2] + 1};
   float norm = bps == 8 ? 255.0f : 65535.0f;
   v->min_value = vmin / norm;
@@ -832,13 +897,13 @@ ASC_API int asc_volume_destroy(asc_volume vol)
   if (!v) return ASC_ERR_ARG;
   Gate g(device_gate());
   cudaFree(v->pairs);
-  if (v->occ) cudaFree(v->occ);
+  if (v->clr) cudaFree(v->clr);
   delete v;
   return ASC_OK;
 }
 
 namespace asc {
-int raycast_launch(const DevVolume& V, const uint8_t* occ, const float* m12, const float* vp, float step,
+int raycast_launch(const DevVolume& V, const uint8_t* clr, const float* m12, const float* vp, float step,
                    float intensity, float cutoff, float* out, int w, int h, cudaStream_t s)
 {
   RayArgs a;
@@ -850,15 +915,8 @@ int raycast_launch(const DevVolume& V, const uint8_t* occ, const float* m12, con
   a.cut = make_cutoff(cutoff, V.norm, V.gmax);
   df_split((double)vp[2] / (double)w, a.sx[0], a.sx[1]);
   df_split((double)vp[3] / (double)h, a.sy[0], a.sy[1]);
-  dim3 grid((w + 15) / 16, (h + 15) / 16);
-  if (V.storage == ASC_STORE_F32)
-    k_raycast<ASC_STORE_F32><<<grid, 256, 0, s>>>(V, occ, a, out, w, h);
-  else if (V.storage == ASC_STORE_BF16)
-    k_raycast<ASC_STORE_BF16><<<grid, 256, 0, s>>>(V, occ, a, out, w, h);
-  else if (V.storage == ASC_STORE_F16)
-    k_raycast<ASC_STORE_F16><<<grid, 256, 0, s>>>(V, occ, a, out, w, h);
-  else
-    k_raycast<ASC_STORE_U16><<<grid, 256, 0, s>>>(V, occ, a, out, w, h);
+  dim3 grid((w + RTX - 1) / RTX, (h + RTY - 1) / RTY);
+  k_raycast<<<grid, NRAY, 0, s>>>(V, clr, a, out, w, h);
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }
@@ -877,21 +935,21 @@ ASC_API int asc_raycast(asc_volume vol, const double imv[16], const float vp[4],
   }
   float m[12];
   fold_matrix(imv, v->inv_scale, v->inv_trans, m);
-  const uint8_t* occ = nullptr;
+  const uint8_t* clr = nullptr;
   if (g_empty_skip) {
     const float cut = occupancy_threshold(make_cutoff(cutoff, v->dev.norm, v->dev.gmax));
-    if (!v->occ) {
+    if (!v->clr) {
       Gate g(device_gate());
-      ASC_CUDA(cudaMalloc(&v->occ, occ_grid_bytes(occupancy_cells(v->dev))));
+      ASC_CUDA(cudaMalloc(&v->clr, clearance_cells(v->dev)));
     }
-    if (!(v->occ_cutoff == cut)) {
-      build_occupancy(v->dev, cut, v->occ, S(stream));
-      ASC_LAUNCH_CHECK();
-      v->occ_cutoff = cut;
+    if (!(v->clr_cutoff == cut)) {
+      int rc = build_clearance(v->dev, cut, v->clr, S(stream));
+      if (rc) return rc;
+      v->clr_cutoff = cut;
     }
-    occ = v->occ;
+    clr = v->clr;
   }
-  return raycast_launch(v->dev, occ, m, vp, step, intensity, cutoff, out, w, h, S(stream));
+  return raycast_launch(v->dev, clr, m, vp, step, intensity, cutoff, out, w, h, S(stream));
 }
 
 // ---- images ----

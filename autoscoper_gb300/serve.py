@@ -72,11 +72,11 @@ VOXEL_BYTES = 8  # two x-pair words (rows y and y+1) per padded voxel
 
 
 def volume_bytes(vol: S.Volume) -> int:
-    """Device bytes of a volume: the padded voxel words plus its occupancy
-    grids (a byte and a 16-byte box per 8^3 cell, one grid per view)."""
+    """Device bytes of a volume: the padded voxel words plus its clearance
+    grids (a byte per 2^3 cell, one grid per view)."""
     D, H, W = vol.data.shape
-    cells = ((W + 7) // 8 + 4) * ((H + 7) // 8 + 4) * ((D + 7) // 8 + 4)
-    return VOXEL_BYTES * (W + 2 * PAD) * (H + 2 * PAD) * (D + 2 * PAD) + 3 * 17 * cells
+    cells = ((W + 1) // 2) * ((H + 1) // 2) * ((D + 1) // 2)
+    return VOXEL_BYTES * (W + 2 * PAD) * (H + 2 * PAD) * (D + 2 * PAD) + 3 * cells
 
 
 def job_bytes(job: Job) -> int:
@@ -85,11 +85,12 @@ def job_bytes(job: Job) -> int:
 
 
 def engine_bytes(n_views: int, rw: int, rh: int, max_items: int, slots: int = 4) -> int:
-    """Device bytes asc_engine_create reserves: DRR crops, tile partials,
-    layouts, the plain-path buffers."""
+    """Device bytes asc_engine_create reserves: DRR crops, tile partials, ray
+    tile and beam lists, layouts, the plain-path buffers."""
     n_iv = max_items * min(slots, n_views)
     tiles = ((rw + 47) // 48) * ((rh + 47) // 48)
-    return n_iv * rw * rh * 4 + n_iv * tiles * 72 + 7 * rw * rh * 4 + n_iv * 200 + max_items * 80
+    ray_tiles = ((rw + 15) // 16) * ((rh + 15) // 16)
+    return n_iv * (rw * rh * 4 + tiles * 76 + ray_tiles * 36 + 200) + 7 * rw * rh * 4 + max_items * 80
 
 
 class VolumeCache:

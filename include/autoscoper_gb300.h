@@ -50,8 +50,7 @@ typedef struct asc_image_s *asc_image;
 typedef struct asc_engine_s *asc_engine;
 
 /* Options (asc_set_option).  ASC_OPT_EMPTY_SKIP (default 1): the ray march
- * steps over runs of samples inside 8^3-voxel cells whose voxels are all at
- * or below the cutoff.  Such samples add exactly nothing in the reference
+ * steps over runs of samples that touch no voxel above the cutoff.  Such samples add exactly nothing in the reference
  * (RayCaster_kernels.cu:189), so results are identical either way; 0 reads
  * every sample (for A/B checks). */
 #define ASC_OPT_EMPTY_SKIP 1
@@ -317,8 +316,10 @@ int asc_engine_stats(asc_engine e, float ms[3], unsigned long long *samples, uns
 /* Ray-cast work counters of the last evaluation: out[0] trilinear samples of
  * the reference's march (far to near over the whole box), out[1] pixels,
  * out[2] samples actually marched after empty-space skipping, out[3] lane
- * slots the marching warps occupied (32 x the longest marched span of each
- * warp's rays); out[2] / out[3] is the SIMT efficiency of the march. */
+ * slots the marching warps occupied (32 x the longest segment of each warp's
+ * rays, over the segments it marches side by side); out[2] / out[3] is the
+ * SIMT efficiency of the march.  out[0] is counted when it is asked for, from
+ * the evaluation's own records. */
 int asc_engine_counters(asc_engine e, unsigned long long out[4]);
 /* Rays of the last evaluation that the ray cast marched a second time: rays
  * with a sample whose FP32 value lay within rounding of the cutoff, whose

@@ -2,11 +2,11 @@
 // for many (bone, manipulator) candidates per pass, with the scene resident
 // on the device.
 //
-// One evaluation is six launches on one stream (seven with cf_model 1):
-//   k_setup_iv    a thread per (item, view): FP64 pose composition, view
-//                            matrix, viewport (Tracker.cpp:603-634) and crop;
-//   k_setup       1 block:  the tile layout of every crop, with prefix sums;
-//   k_tile_map    grid-stride: each ray and view tile's (item, view);
+// One evaluation is four launches on one stream (five with cf_model 1):
+//   k_setup       a warp per item: FP64 pose composition, view matrices,
+//                            viewports (Tracker.cpp:603-634) and crops; the
+//                            last block: the tile layout of every crop, with
+//                            prefix sums and each tile's (item, view);
 //   k_ray         persistent: a warp per beam of 32 rays from an atomic
 //                            queue, DRRs written to a packed buffer; rays
 //                            with a sample within rounding of the cutoff are
@@ -119,7 +119,7 @@ struct Counters {
   int error;
   int nfix;   // rays whose march met the cutoff's band (k_ray_fix marches them again)
   int nfixb;  // beams holding such rays
-  int pad;
+  unsigned setup;  // blocks of k_setup done; 0 between evaluations
   unsigned long long samples, pixels;
   unsigned long long marched, slots;  // marched samples, 32 x warp-max span
 };
@@ -137,20 +137,10 @@ struct Bufs {
   unsigned* ivt;   // per-iv tile tickets
   unsigned* itt;   // per-item view tickets
   unsigned* fixb;  // beams (ray tile x BEAMS + its beam) holding rays to march again exactly (k_ray_fix)
-  int* rtile_iv;   // per ray tile: its (item, view) (k_tile_map)
+  int* rtile_iv;   // per ray tile: its (item, view) (k_setup)
   int* ftile_iv;   // per view tile: its (item, view)
   Counters* C;
 };
-
-__device__ __forceinline__ int find_iv(const int* off, int n, int tile)
-{
-  int lo = 0, hi = n;  // off[lo] <= tile < off[hi]
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (__ldg(off + mid) <= tile) lo = mid; else hi = mid;
-  }
-  return lo;
-}
 
 __device__ void finish_item(const SceneDev* sc, const Bufs& b, int item, double* cost)
 {
@@ -160,154 +150,399 @@ __device__ void finish_item(const SceneDev* sc, const Bufs& b, int item, double*
 }
 
 // ---------------------------------------------------------------- k_setup
-// One (item, view) of trackFrame's set-up: the pose (minimizationFunc), the
-// folded matrix, the viewport and crop size, its ray and view tile counts.
-__device__ void setup_iv(const SceneDev* __restrict__ sc, int k, const int* __restrict__ bone_in,
-                         const double* __restrict__ manip, const Bufs& b)
+// The FP64 set-up of an item (minimizationFunc's pose, then trackFrame's
+// view matrix, viewport and crop for each of its views) by one warp, its
+// intermediate frames in the warp's shared memory.  An FP64 operation takes
+// a warp 16 issue cycles and its dependants ~40 whatever its active lanes, so
+// what counts is the chain's length: the sines, the elements of a rotation
+// or product, the volume's corners and the quotients are dealt to lanes, and
+// the operands and the order of each stay those of frame_* (asc_internal.cuh).
+constexpr int SETUP_THREADS = 256;
+struct SetupWarp {
+  double f[2][12];     // frames under construction (rotations, translation)
+  double R[2][9];      // their next rotation
+  double t[3][12];     // products
+  double mv[4][12], imv[4][12];  // per view
+  double film[4][4], corner[4][6];  // per view: the image's film-plane box, the volume's faces (setup_view)
+};
+
+// frame_rotate of f[side] about a by the angle of cosine c and sine s, by 16
+// lanes per side; `on`: this side takes part.
+__device__ __forceinline__ void warp_rotate(SetupWarp& w, int side, int e, bool on, double a0, double a1, double a2,
+                                            double c, double s)
 {
-  const int ns = sc->slots;
-  const int item = k / ns, j = k % ns;
-  IV r;
-  memset(&r, 0, sizeof r);
-  int bi = bone_in[item];
-  if (bi < 0 || bi >= sc->n_bones) bi = 0;
+  const double mag = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
+  const double mine = (e % 3 == 0 ? a0 : (e % 3 == 1 ? a1 : a2)) / mag;
+  const int first = (threadIdx.x & 16);
+  a0 = __shfl_sync(FULL_WARP, mine, first);
+  a1 = __shfl_sync(FULL_WARP, mine, first + 1);
+  a2 = __shfl_sync(FULL_WARP, mine, first + 2);
+  on = on && mag != 0 && e < 9;
+  const int i = e / 3, j = e % 3;
+  const double oc = 1.0 - c;
+  if (on) {
+    // row-vector rotation matrix: oc a_i a_j, plus c on the diagonal, plus or
+    // minus s a_k off it
+    const int lo = min(i, j), hi = max(i, j), k = 3 - lo - hi;
+    const double al = lo == 0 ? a0 : (lo == 1 ? a1 : a2), ah = hi == 0 ? a0 : (hi == 1 ? a1 : a2);
+    const double ak = k == 0 ? a0 : (k == 1 ? a1 : a2);
+    const bool plus = (j - i + 3) % 3 == 1;  // (0,1), (1,2), (2,0)
+    w.R[side][e] = i == j ? oc * al * al + c : oc * al * ah + (plus ? s : -s) * ak;
+  }
+  __syncwarp();
+  double t = 0.0;
+  if (on) {
+    const double *f = w.f[side] + 3 * i, *R = w.R[side] + j;
+    t = f[0] * R[0] + f[1] * R[3] + f[2] * R[6];
+  }
+  __syncwarp();
+  if (on) w.f[side][e] = t;
+  __syncwarp();
+}
+
+// out = a . b (frame_mul), an element per lane.
+__device__ __forceinline__ void warp_mul(const double* a, const double* b, double* out, int lane)
+{
+  if (lane < 12) {
+    const int c = lane / 3, i = lane % 3;
+    const double r = a[i] * b[3 * c] + a[3 + i] * b[3 * c + 1] + a[6 + i] * b[3 * c + 2];
+    out[lane] = c == 3 ? r + a[9 + i] : r;
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ double shfl_min(double v, int o) { return fmin(v, __shfl_xor_sync(FULL_WARP, v, o)); }
+__device__ __forceinline__ double shfl_max(double v, int o) { return fmax(v, __shfl_xor_sync(FULL_WARP, v, o)); }
+
+// What an item's views need besides its pose, by a second warp meanwhile: 8
+// lanes per view, the corners of its image in the film plane
+// (calculate_viewport's rf) and the faces of the bone's box.
+__device__ __forceinline__ void setup_view(const SceneDev* __restrict__ sc, int bi, SetupWarp& w)
+{
+  const BoneDev& B = sc->bones[bi];
+  const int lane = threadIdx.x & 31, j = lane >> 3, l = lane & 7, first = lane & ~7;
+  const ViewDev& V = sc->views[j < sc->slots && j < B.n_slots ? B.view_of[j] : 0];
+  const int i = l % 3;
+  const double *a = V.cam, *p = V.ip + (l < 3 ? 3 : 9);
+  const double at = -(a[3 * i] * a[9] + a[3 * i + 1] * a[10] + a[3 * i + 2] * a[11]);
+  const double q = a[3 * i] * p[0] + a[3 * i + 1] * p[1] + a[3 * i + 2] * p[2] + at;
+  const double num = __shfl_sync(FULL_WARP, q, first + (l < 2 ? l : (l < 4 ? l + 1 : 0)));
+  const double den = __shfl_sync(FULL_WARP, q, first + (l < 2 ? 2 : 5));
+  if (l < 4) w.film[j][l] = -2 * num / den;
+  if (l < 6) {
+    const int k = l >> 1;
+    const double face = k < 2 ? (double)(l & 1) : (double)(l & 1) - 1.0;
+    w.corner[j][l] = (face - (double)B.inv_trans[k]) / (double)B.inv_scale[k];
+  }
+}
+
+// The frame of yaw (cosine c, sine s) about z alone, what frame_rotate makes
+// of the identity.
+__device__ __forceinline__ void warp_yaw(double* f, int lane, double c, double s)
+{
+  if (lane < 12) {
+    const double one = 1.0 - c + c;
+    f[lane] = lane == 0 || lane == 4 ? c : (lane == 1 ? s : (lane == 3 ? -s : (lane == 8 ? one : 0.0)));
+  }
+  __syncwarp();
+}
+
+// The item's pose: its frame into w.f[0].
+__device__ void setup_pose(const SceneDev* __restrict__ sc, int item, int bi, const double* __restrict__ manip,
+                           SetupWarp& w)
+{
+  const double PI = 3.14159265358979323846;
+  const int lane = threadIdx.x & 31, side = lane >> 4, e = lane & 15;
+  const BoneDev& B = sc->bones[bi];
+  const double* man = manip + 6 * item;
+  // ---- minimizationFunc: pose . V^-1 . manip . V, then the xyzypr round trip.
+  // side 0: the base pose's frame; side 1: the manipulator's
+  const double v3 = man[3], v4 = man[4], v5 = man[5];
+  const double ang = sqrt(v3 * v3 + v4 * v4 + v5 * v5);
+  double c, s;
+  sincos(PI * (lane < 3 ? B.base[3 + lane] : ang) / 180.0, &s, &c);
+  warp_yaw(w.f[0], lane, __shfl_sync(FULL_WARP, c, 0), __shfl_sync(FULL_WARP, s, 0));
+  if (side == 1 && e < 12) w.f[1][e] = e == 0 || e == 4 || e == 8 ? 1.0 : 0.0;
+  __syncwarp();
+  for (int k = 1; k < 3; ++k) {  // pitch about the new y, roll about the new x
+    const double* ax = w.f[0] + 6 - 3 * k;
+    const double a0 = side ? v3 : ax[0], a1 = side ? v4 : ax[1], a2 = side ? v5 : ax[2];
+    const int from = side ? 3 : k;
+    const double ck = __shfl_sync(FULL_WARP, c, from), sk = __shfl_sync(FULL_WARP, s, from);
+    warp_rotate(w, side, e, side == 0 || (k == 1 && ang != 0), a0, a1, a2, ck, sk);
+  }
+  if (lane < 3) w.f[0][9 + lane] += B.base[lane];
+  if (side == 1 && e < 3) w.f[1][9 + e] += man[e];
+  __syncwarp();
+  warp_mul(w.f[0], B.pivot_inv, w.t[0], lane);
+  warp_mul(w.t[0], w.f[1], w.t[1], lane);
+  warp_mul(w.t[1], B.pivot, w.t[2], lane);
+  {
+    const double* f = w.t[2];
+    const double q = sqrt(f[5] * f[5] + f[8] * f[8]);
+    const double y = lane == 0 ? f[1] : (lane == 1 ? -f[2] : f[5]), x = lane == 0 ? f[0] : (lane == 1 ? q : f[8]);
+    const double ypr = 180.0 * atan2(y, x) / PI;
+    sincos(PI * ypr / 180.0, &s, &c);
+  }
+  warp_yaw(w.f[0], lane, __shfl_sync(FULL_WARP, c, 0), __shfl_sync(FULL_WARP, s, 0));
+  for (int k = 1; k < 3; ++k) {
+    const double* ax = w.f[0] + 6 - 3 * k;
+    const double a0 = ax[0], a1 = ax[1], a2 = ax[2];
+    const double ck = __shfl_sync(FULL_WARP, c, k), sk = __shfl_sync(FULL_WARP, s, k);
+    warp_rotate(w, side, e, side == 0, a0, a1, a2, ck, sk);
+  }
+  if (lane < 3) w.f[0][9 + lane] += w.t[2][9 + lane];
+  __syncwarp();
+}
+
+// trackFrame (1a)-(1c) of the item's views, 8 lanes each.
+__device__ void setup_views(const SceneDev* __restrict__ sc, int item, int bi, const Bufs& b, SetupWarp& w)
+{
+  const int lane = threadIdx.x & 31, ns = sc->slots, j = lane >> 3, l = lane & 7;
+  const BoneDev& B = sc->bones[bi];
+  const bool on = j < ns && j < B.n_slots;  // past the bone's views: a slot that adds nothing to the cost
+  const int view = on ? B.view_of[j] : 0;
+  const ViewDev& V = sc->views[view];
+  double *mv = w.mv[j], *imv = w.imv[j];
+  for (int q = l; q < 12; q += 8) {
+    const int cc = q / 3, i = q % 3;
+    const double *a = V.cam_inv, *t = w.f[0];
+    const double r = a[i] * t[3 * cc] + a[3 + i] * t[3 * cc + 1] + a[6 + i] * t[3 * cc + 2];
+    mv[q] = cc == 3 ? r + a[9 + i] : r;
+  }
+  __syncwarp();
+  for (int q = l; q < 12; q += 8) {  // frame_inverse
+    const int cc = q / 3, i = q % 3;
+    imv[q] = cc < 3 ? mv[3 * i + cc] : -(mv[3 * i] * mv[9] + mv[3 * i + 1] * mv[10] + mv[3 * i + 2] * mv[11]);
+  }
+  const int first = lane & ~7;
+  // calculate_viewport, the volume's corners a lane each
+  const double rf0 = w.film[j][0], rf1 = w.film[j][1], rf2 = w.film[j][2], rf3 = w.film[j][3];
+  double lo0, lo1, hi0, hi1;
+  {
+    const double p0 = w.corner[j][l >> 2], p1 = w.corner[j][2 + (l >> 1 & 1)], p2 = w.corner[j][4 + (l & 1)];
+    double q[3];
+    for (int i = 0; i < 3; ++i) q[i] = mv[i] * p0 + mv[3 + i] * p1 + mv[6 + i] * p2 + mv[9 + i];
+    const double fx = -2 * q[0] / q[2], fy = -2 * q[1] / q[2];
+    lo0 = fmin(1.0, fx);
+    lo1 = fmin(1.0, fy);
+    hi0 = fmax(-1.0, fx);
+    hi1 = fmax(-1.0, fy);
+  }
+  for (int o = 1; o < 8; o <<= 1) {
+    lo0 = shfl_min(lo0, o);
+    lo1 = shfl_min(lo1, o);
+    hi0 = shfl_max(hi0, o);
+    hi1 = shfl_max(hi1, o);
+  }
+  __syncwarp();  // imv
+  const bool seen = !((lo0 > rf2 && hi0 > rf2) || (lo1 > rf3 && hi1 > rf3) || (lo0 < rf0 && hi0 < rf0) ||
+                      (lo1 < rf1 && hi1 < rf1) || (lo0 == 1.0 && lo1 == 1.0 && hi0 == -1.0 && hi1 == -1.0));
+  if (lo0 < rf0) lo0 = rf0;
+  if (lo1 < rf1) lo1 = rf1;
+  if (hi0 > rf2) hi0 = rf2;
+  if (hi1 > rf3) hi1 = rf3;
+  const double vp2 = hi0 - lo0, vp3 = hi1 - lo1;
+  // the crop's width (even lanes) and height (odd lanes), and its pixels' spacing
+  const bool odd = l & 1;
+  const double fs = (odd ? vp3 : vp2) * (odd ? V.rh : V.rw) / V.cvp[odd ? 3 : 2];
+  unsigned n = fs > 0 ? (unsigned)fs : 0u;
+  float sh = 0.f, sl = 0.f;
+  const double spacing = (double)(float)(odd ? vp3 : vp2) / (double)n;
+  if (n > 0) df_split(spacing, sh, sl);
+  unsigned cw = __shfl_sync(FULL_WARP, n, first), ch = __shfl_sync(FULL_WARP, n, first + 1);
+  const float syh = __shfl_sync(FULL_WARP, sh, first + 1), syl = __shfl_sync(FULL_WARP, sl, first + 1);
+  if (j >= ns) return;
+  const int k = item * ns + j;
+  IV& r = b.iv[k];
+  if (on)
+    for (int q = l; q < 12; q += 8) {  // fold_matrix
+      const int row = q / 4, cc = q % 4;
+      const double last = cc < 3 ? 0.0 : 1.0;
+      r.m[q] = (float)(imv[cc < 3 ? 3 * cc + row : 9 + row] * (double)B.inv_scale[row] + last * (double)B.inv_trans[row]);
+    }
+  if (l != 0) return;
   r.bone = bi;
   r.slot = j;
-  const BoneDev& B = sc->bones[bi];
-  if (j >= B.n_slots) {  // a slot this bone has no view in: adds nothing to the cost
-    r.view = -1;
-    b.iv[k] = r;
-    b.vcost[k] = 0.0;
-    b.ivt[k] = 0;
-    return;
-  }
-  const int v = B.view_of[j];
-  r.view = v;
-  const ViewDev& V = sc->views[v];
-  // minimizationFunc: pose . V^-1 . manip . V, then the xyzypr round trip
-  double base[12], man[12], t1[12], t2[12], xyz[6];
-  frame_from_xyzypr(B.base, base);
-  frame_from_axis_angle(manip + 6 * item, man);
-  frame_mul(base, B.pivot_inv, t1);
-  frame_mul(t1, man, t2);
-  frame_mul(t2, B.pivot, t1);
-  frame_to_xyzypr(t1, xyz);
-  frame_from_xyzypr(xyz, t1);
-  // trackFrame (1a)-(1c)
-  double mv[12], imv[12], imv16[16], vp[4];
-  frame_mul(V.cam_inv, t1, mv);
-  frame_inverse(mv, imv);
-  frame_row_matrix(imv, imv16);
-  fold_matrix(imv16, B.inv_scale, B.inv_trans, r.m);
-  const Cutoff& cut = B.cut[j];
-  r.band[0] = cut.raw - cut.t0;
-  r.band[1] = cut.hi0 + cut.t0;
-  r.band[2] = cut.t1;
-  r.step = B.step[j];
-  r.nx = B.vol.nx;
-  r.ny = B.vol.ny;
-  r.nz = B.vol.nz;
+  r.view = on ? view : -1;
+  r.w = r.h = r.ok = r.err = 0;
+  r.rtx = r.rty = r.ftx = r.fty = 0;
   double vc = 0.0;
-  if (!calculate_viewport(mv, V.cam, V.ip, B.inv_scale, B.inv_trans, vp)) {
-    vc = 9999.0;  // Tracker.cpp:614-617
-  } else {
-    double fw = vp[2] * V.rw / V.cvp[2], fh = vp[3] * V.rh / V.cvp[3];
-    unsigned w = fw > 0 ? (unsigned)fw : 0u, h = fh > 0 ? (unsigned)fh : 0u;
-    if (w > (unsigned)V.rw || h > (unsigned)V.rh) {
-      r.err = 1;  // the reference throws (Tracker.cpp:625-629)
-      w = 0;
-      h = 0;
-    }
-    r.w = (int)w;
-    r.h = (int)h;
-    for (int j = 0; j < 4; ++j) r.vp[j] = (float)vp[j];
-    if (w > 0 && h > 0) {
-      df_split((double)r.vp[2] / (double)w, r.sx[0], r.sx[1]);
-      df_split((double)r.vp[3] / (double)h, r.sy[0], r.sy[1]);
-    }
-    if (w == 0 || h == 0 || !B.visible) {
-      // an empty crop, or the all-zero DRR of a hidden volume (RayCaster.cpp:131-134),
-      // whose mask is empty: the degenerate NCC (1e5), or the SAD of no pixels
-      vc = sc->cf_model ? 0.0 : 1.0 - 1e5;
+  if (on) {
+    const Cutoff& cut = B.cut[j];
+    r.band[0] = cut.raw - cut.t0;
+    r.band[1] = cut.hi0 + cut.t0;
+    r.band[2] = cut.t1;
+    r.step = B.step[j];
+    r.nx = B.vol.nx;
+    r.ny = B.vol.ny;
+    r.nz = B.vol.nz;
+    if (!seen) {
+      vc = 9999.0;  // Tracker.cpp:614-617
     } else {
-      r.ok = 1;
-      r.rtx = (r.w + RTX - 1) / RTX;
-      r.rty = (r.h + RTY - 1) / RTY;
-      r.ftx = (r.w + VT - 1) / VT;
-      r.fty = (r.h + VT - 1) / VT;
+      if (cw > (unsigned)V.rw || ch > (unsigned)V.rh) {
+        r.err = 1;  // the reference throws (Tracker.cpp:625-629)
+        cw = 0;
+        ch = 0;
+      }
+      r.w = (int)cw;
+      r.h = (int)ch;
+      r.vp[0] = (float)lo0;
+      r.vp[1] = (float)lo1;
+      r.vp[2] = (float)vp2;
+      r.vp[3] = (float)vp3;
+      r.sx[0] = sh;
+      r.sx[1] = sl;
+      r.sy[0] = syh;
+      r.sy[1] = syl;
+      if (cw == 0 || ch == 0 || !B.visible) {
+        // an empty crop, or the all-zero DRR of a hidden volume (RayCaster.cpp:131-134),
+        // whose mask is empty: the degenerate NCC (1e5), or the SAD of no pixels
+        vc = sc->cf_model ? 0.0 : 1.0 - 1e5;
+      } else {
+        r.ok = 1;
+        r.rtx = (r.w + RTX - 1) / RTX;
+        r.rty = (r.h + RTY - 1) / RTY;
+        r.ftx = (r.w + VT - 1) / VT;
+        r.fty = (r.h + VT - 1) / VT;
+      }
     }
   }
-  b.iv[k] = r;
   b.vcost[k] = vc;
   b.ivt[k] = 0;
 }
 
-// Every (item, view) at once: the FP64 set-up of each runs on its own thread
-// across the GPU.
-__global__ void __launch_bounds__(128) k_setup_iv(const SceneDev* __restrict__ sc, int n_items,
-                                                  const int* __restrict__ bone_in, const double* __restrict__ manip,
-                                                  Bufs b)
+// Exclusive sums over the block's threads of a, c and p, and their totals
+// (s: 3 words of 8 bytes per warp).
+__device__ __forceinline__ void block_scan3(int& a, int& c, long long& p, int& ta, int& tc, long long& tp,
+                                            long long (*s)[SETUP_THREADS / 32])
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n_items * sc->slots) setup_iv(sc, k, bone_in, manip, b);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int ia = a, ic = c;
+  long long ip = p;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ua = __shfl_up_sync(FULL_WARP, ia, o), uc = __shfl_up_sync(FULL_WARP, ic, o);
+    const long long up = __shfl_up_sync(FULL_WARP, ip, o);
+    if (lane >= o) {
+      ia += ua;
+      ic += uc;
+      ip += up;
+    }
+  }
+  __syncthreads();
+  if (lane == 31) {
+    s[0][warp] = ia;
+    s[1][warp] = ic;
+    s[2][warp] = ip;
+  }
+  __syncthreads();
+  ta = tc = 0;
+  tp = 0;
+  int ba = 0, bc = 0;
+  long long bp = 0;
+  for (int q = 0; q < SETUP_THREADS / 32; ++q) {
+    if (q == warp) {
+      ba = ta;
+      bc = tc;
+      bp = tp;
+    }
+    ta += (int)s[0][q];
+    tc += (int)s[1][q];
+    tp += s[2][q];
+  }
+  a = ba + ia - a;
+  c = bc + ic - c;
+  p = bp + ip - p;
 }
 
-// The layout of a batch after k_setup_iv: prefix sums of the tile counts and
-// crop sizes (ray tiles, view tiles, DRR offsets), the batch counters, and
-// the items' view tickets (views finished in set-up count as arrived).
-__global__ void __launch_bounds__(1024) k_setup(const SceneDev* __restrict__ sc, int n_items, Bufs b,
-                                                 double* __restrict__ cost)
+// p[from, to) = v by a warp, 16 bytes a lane between the ends.
+__device__ __forceinline__ void warp_fill(int* __restrict__ p, int from, int to, int v, int lane)
 {
+  const int a = min((from + 3) & ~3, to), z = max(a, to & ~3);
+  if (from + lane < a) p[from + lane] = v;
+  for (int t = a + 4 * lane; t < z; t += 128) *(int4*)(p + t) = make_int4(v, v, v, v);
+  if (z + lane < to) p[z + lane] = v;
+}
+
+// Every item's set-up, by one warp of its block (the SM's FP64 unit serves
+// one at a time, a second warp the part that needs no pose); then the last block to finish lays the batch out: prefix sums of the tile counts and crop sizes (ray tiles, view
+// tiles, DRR offsets), each tile's (item, view), so that the persistent
+// kernels look a grabbed tile up with one load, the batch counters, and the
+// items' view tickets (views finished here count as arrived).
+// What bounds it is the latency of one FP64 chain (~70 cycles an operation).
+// One thread per (item, view) took 78 us, with two launches after it for the
+// layout and the tile map: 88 us for 4 candidates, 99 for 300; here 28 and 74.
+__global__ void __launch_bounds__(SETUP_THREADS) k_setup(const SceneDev* __restrict__ sc, int n_items,
+                                                         const int* __restrict__ bone_in,
+                                                         const double* __restrict__ manip, Bufs b,
+                                                         double* __restrict__ cost)
+{
+  __shared__ SetupWarp s_w;
+  __shared__ long long s_scan[3][SETUP_THREADS / 32];
+  __shared__ int s_ray[SETUP_THREADS + 1], s_view[SETUP_THREADS + 1];
   __shared__ int s_err;
+  __shared__ bool s_last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int bi = bone_in[blockIdx.x];
+  if (bi < 0 || bi >= sc->n_bones) bi = 0;
+  if (warp == 0) setup_pose(sc, blockIdx.x, bi, manip, s_w);
+  if (warp == 1) setup_view(sc, bi, s_w);
+  __syncthreads();
+  if (warp == 0) {
+    setup_views(sc, blockIdx.x, bi, b, s_w);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(&b.C->setup, 1u) == gridDim.x - 1;
+    s_err = 0;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   const int nv = sc->slots, n_iv = n_items * nv;
-  const int per = (n_iv + blockDim.x - 1) / blockDim.x;
-  const int i0 = threadIdx.x * per, i1 = min(i0 + per, n_iv);
-  if (threadIdx.x == 0) s_err = 0;
-  __syncthreads();
-  int rsum = 0, fsum = 0;
-  long long psum = 0;
-  for (int k = i0; k < i1; ++k) {
-    const IV& r = b.iv[k];
-    if (r.err) s_err = ASC_ERR_RANGE;
-    psum += (long long)r.w * r.h;
-    rsum += r.rtx * r.rty;
-    fsum += r.ftx * r.fty;
-  }
-  // block-wide exclusive scan of (rsum, fsum, psum)
-  __shared__ long long sp[1024];
-  __shared__ int sr[1024], sf[1024];
-  sr[threadIdx.x] = rsum;
-  sf[threadIdx.x] = fsum;
-  sp[threadIdx.x] = psum;
-  __syncthreads();
-  for (int o = 1; o < blockDim.x; o <<= 1) {
-    int a = threadIdx.x >= o ? sr[threadIdx.x - o] : 0;
-    int c = threadIdx.x >= o ? sf[threadIdx.x - o] : 0;
-    long long p = threadIdx.x >= o ? sp[threadIdx.x - o] : 0;
+  int ray = 0, view = 0;
+  long long pix = 0;
+  for (int k0 = 0; k0 < n_iv; k0 += SETUP_THREADS) {
+    const int k = k0 + threadIdx.x;
+    int a = 0, c = 0, ta, tc;
+    long long p = 0, tp;
+    if (k < n_iv) {
+      const IV& r = b.iv[k];
+      if (__ldcg(&r.err)) s_err = ASC_ERR_RANGE;
+      a = __ldcg(&r.rtx) * __ldcg(&r.rty);
+      c = __ldcg(&r.ftx) * __ldcg(&r.fty);
+      p = (long long)__ldcg(&r.w) * __ldcg(&r.h);
+    }
+    block_scan3(a, c, p, ta, tc, tp, s_scan);
+    s_ray[threadIdx.x] = ray + a;
+    s_view[threadIdx.x] = view + c;
+    if (k < n_iv) {
+      b.iv[k].pix = pix + p;
+      b.roff[k] = ray + a;
+      b.foff[k] = view + c;
+    }
+    ray += ta;
+    view += tc;
+    pix += tp;
+    if (threadIdx.x == 0) {
+      s_ray[SETUP_THREADS] = ray;
+      s_view[SETUP_THREADS] = view;
+    }
     __syncthreads();
-    sr[threadIdx.x] += a;
-    sf[threadIdx.x] += c;
-    sp[threadIdx.x] += p;
+    for (int q = warp; q < SETUP_THREADS && k0 + q < n_iv; q += SETUP_THREADS / 32) {
+      warp_fill(b.rtile_iv, s_ray[q], s_ray[q + 1], k0 + q, lane);
+      warp_fill(b.ftile_iv, s_view[q], s_view[q + 1], k0 + q, lane);
+    }
     __syncthreads();
   }
-  int rbase = sr[threadIdx.x] - rsum, fbase = sf[threadIdx.x] - fsum;
-  long long pbase = sp[threadIdx.x] - psum;
-  for (int k = i0; k < i1; ++k) {
-    IV& r = b.iv[k];
-    r.pix = pbase;
-    b.roff[k] = rbase;
-    b.foff[k] = fbase;
-    pbase += (long long)r.w * r.h;
-    rbase += r.rtx * r.rty;
-    fbase += r.ftx * r.fty;
-  }
-  if (threadIdx.x == blockDim.x - 1) {
-    b.roff[n_iv] = rbase;
-    b.foff[n_iv] = fbase;
+  if (threadIdx.x == 0) {
+    b.roff[n_iv] = ray;
+    b.foff[n_iv] = view;
     b.C->n_items = n_items;
     b.C->n_iv = n_iv;
-    b.C->rtiles = rbase;
-    b.C->ftiles = fbase;
+    b.C->rtiles = ray;
+    b.C->ftiles = view;
     b.C->rnext = 0;
     b.C->fnext = 0;
     b.C->error = s_err;
@@ -316,30 +551,16 @@ __global__ void __launch_bounds__(1024) k_setup(const SceneDev* __restrict__ sc,
     b.C->samples = 0;
     b.C->marched = 0;
     b.C->slots = 0;
-    b.C->pixels = (unsigned long long)(sp[threadIdx.x]);
+    b.C->pixels = (unsigned long long)pix;
+    b.C->setup = 0;
   }
-  __syncthreads();
   // item tickets: views finished here count as arrived
   for (int item = threadIdx.x; item < n_items; item += blockDim.x) {
     unsigned pre = 0;
-    for (int v = 0; v < nv; ++v) pre += b.iv[item * nv + v].ok ? 0u : 1u;
+    for (int v = 0; v < nv; ++v) pre += __ldcg(&b.iv[item * nv + v].ok) ? 0u : 1u;
     b.itt[item] = pre;
     if (pre == (unsigned)nv) finish_item(sc, b, item, cost);
   }
-}
-
-// Every ray tile's and view tile's (item, view), so that the persistent
-// kernels look a grabbed tile up with one load instead of a binary search
-// over the prefix sums (ten dependent loads while the block waits).
-// (Dealing most ray tiles to the blocks in turn, with a queue for the rest,
-// measured 9 % slower: a block then owns fixed columns of every crop, and the
-// central ones cost more.)
-__global__ void __launch_bounds__(256) k_tile_map(Bufs b)
-{
-  const int rt = b.C->rtiles, ft = b.C->ftiles, n = b.C->n_iv;
-  const int stride = gridDim.x * blockDim.x;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < rt; t += stride) b.rtile_iv[t] = find_iv(b.roff, n, t);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ft; t += stride) b.ftile_iv[t] = find_iv(b.foff, n, t);
 }
 
 // ---------------------------------------------------------------- k_ray
@@ -1649,9 +1870,7 @@ static int engine_launch(asc_engine e, int n, const int* bone, const double* man
 {
   const bool prof = e->prof && !capturing;
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[0], s));
-  k_setup_iv<<<(n * e->host.slots + 127) / 128, 128, 0, s>>>(e->dev, n, bone, manip, e->b);
-  k_setup<<<1, 1024, 0, s>>>(e->dev, n, e->b, cost);
-  k_tile_map<<<e->sms * 2, 256, 0, s>>>(e->b);
+  k_setup<<<n, SETUP_THREADS, 0, s>>>(e->dev, n, bone, manip, e->b, cost);
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[1], s));
   k_ray<<<e->sms * e->launch.ray_blocks_per_sm, NRAY, 0, s>>>(e->dev, e->b, g_empty_skip, e->launch.ray_shape);
   k_ray_fix<<<e->sms * 4, FIX_THREADS, 0, s>>>(e->dev, e->b, e->launch.ray_shape);

@@ -65,7 +65,6 @@ struct ViewDev {
   double cam[12], cam_inv[12], ip[12], cvp[4];
   float ipf[4];
   int rw, rh;  // render size of this view's trial (Trial::render_width/height)
-  int E;       // k_view region edge: VT + 2 x the larger chain halo
   const void* rad;
   int rad_w, rad_h, rad_bps;
   const float* bg;
@@ -90,7 +89,7 @@ struct BoneDev {
 };
 
 struct SceneDev {
-  int n_views, n_bones, rw, rh, coverage, E;  // rw, rh, E: the largest of the views'
+  int n_views, n_bones, rw, rh, coverage, halo;  // rw, rh, halo: the largest of the views'
   int slots;     // (item, slot) entries per item: the most views a bone is scored in
   int cf_model;  // 0: 1 - NCC per view; 1: SAD ("hdist") per view
   ViewDev views[MAX_VIEWS];
@@ -669,12 +668,13 @@ __global__ void __launch_bounds__(NRAY) k_count_samples(Bufs b)
 }
 
 // ---------------------------------------------------------------- k_view
-// Region coordinates: buffer index (ry, rx) <-> image (y0 + ry, x0 + rx) with
-// x0 = tile x - E_h, where E_h = (E - VT) / 2 is the largest chain halo.
-// `in` is set when the whole E x E region lies inside the image: the stages
-// then skip every bounds test.
+// A tile's region: region column rx, row ry <-> image (x0 + rx, y0 + ry),
+// rows `P` floats apart.  The tile starts at column EX (a multiple of 4, so
+// that four columns of the tile are 16 aligned bytes in every buffer) and row
+// EY, the larger chain's halo.  `in`: the region that the chains read lies
+// inside the image, and the stages skip every bounds test.
 struct Region {
-  int x0, y0, E, w, h;
+  int x0, y0, P, EX, EY, w, h;
   bool in;
 };
 
@@ -684,21 +684,30 @@ __device__ __forceinline__ bool inside(const Region& g, int ry, int rx)
   return x >= 0 && x < g.w && y >= 0 && y < g.h;
 }
 
-// Calls f(ry, rx) for every position of the band [y0, y1) x [x0, x1), the
-// positions dealt to the block's threads in row-major order (consecutive
-// threads take consecutive columns, wrapping to the next row), so no lane
-// idles on bands narrower or wider than a warp.
-template <class F>
-__device__ __forceinline__ void for_band(int y0, int y1, int x0, int x1, F&& f)
+// A band of the region: the tile and `halo` pixels around it.
+struct Band {
+  int x0, x1, y0, y1;
+};
+__device__ __forceinline__ Band band(const Region& g, int halo)
 {
-  const int bw = x1 - x0, n = bw * (y1 - y0);
+  return Band{g.EX - halo, g.EX + VT + halo, g.EY - halo, g.EY + VT + halo};
+}
+
+// Calls f(ry, rx) for every position of a band, the positions dealt to the
+// block's threads in row-major order (consecutive threads take consecutive
+// columns, wrapping to the next row), so no lane idles on bands narrower or
+// wider than a warp.
+template <class F>
+__device__ __forceinline__ void for_band(const Band& b, F&& f)
+{
+  const int bw = b.x1 - b.x0, n = bw * (b.y1 - b.y0);
   if (bw <= 0 || n <= 0) return;
   const int dq = VNT / bw, dr = VNT - dq * bw;
   int ry = (int)threadIdx.x / bw;
   int rx = (int)threadIdx.x - ry * bw;
-  ry += y0;
+  ry += b.y0;
   for (int i = threadIdx.x; i < n; i += VNT) {
-    f(ry, x0 + rx);
+    f(ry, b.x0 + rx);
     rx += dr;
     ry += dq;
     if (rx >= bw) {
@@ -707,6 +716,22 @@ __device__ __forceinline__ void for_band(int y0, int y1, int x0, int x1, F&& f)
     }
   }
 }
+
+// Calls f(ry, rx) for units of 4 columns of a row of a band (aligned, so up to
+// 3 columns past the band on either side, whose results are not used), dealt
+// to the threads in row-major order.  A unit is one row: taller ones load
+// less, but their unrolled code runs once or twice a tile and waits for
+// the instruction cache (units of 4 rows: 3.71 ms on 300 candidates x 2 views
+// of 1024^2 with the four-filter chain, against 2.84).
+template <class F>
+__device__ __forceinline__ void for_units(const Band& b, F&& f)
+{
+  const int c0 = b.x0 >> 2;
+  for_band(Band{c0, (b.x1 + 3) >> 2, b.y0, b.y1}, [&](int ry, int c) { f(ry, c << 2); });
+}
+
+__device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float part(const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 
 // axy^e1 * v^e2 of ContrastFilter_kernels.cu (two powf there) as one exp2 of
 // the summed logarithms; axy > 0.01 here.  v^0 is 1 for every v, as powf's.
@@ -717,124 +742,142 @@ __device__ __forceinline__ float contrast_pow(float axy, float v, float e1, floa
   return exp2f(l);
 }
 
-// Calls f(ry, rx, nr) for column units: column rx of the band [y0, y1) x
-// [x0, x1), rows ry .. ry + nr - 1 (nr <= VR), consecutive threads taking
-// consecutive columns.  A unit reads a few rows past the band; those reads
-// stay inside the block's shared memory (VR rows of slack follow the
-// buffers) and their results are discarded.
-constexpr int VR = 4;
-
-// k_view's dynamic shared memory, in 4-byte words: three E x E stage
-// buffers, the VT x VT tile, VR + 2 rows of slack for the column units'
-// reads past a band, then the region's per-column and per-row radiograph
-// mapping (texel index and weight each).
-__host__ __device__ constexpr size_t view_tail_floats(int E)
+__device__ __forceinline__ float contrast_px(float axy, float v, float e1, float e2)
 {
-  return (size_t)3 * E * E + (size_t)VT * VT + (size_t)(VR + 2) * E;
+  return axy > 0.01f ? contrast_pow(axy, v, e1, e2) : 0.0f;
 }
-__host__ __device__ constexpr size_t view_smem_floats(int E) { return view_tail_floats(E) + (size_t)4 * E; }
-constexpr int kNoTexel = -0x7fffffff;  // a column or row that maps outside the radiograph
-template <class F>
-__device__ __forceinline__ void for_units(int y0, int y1, int x0, int x1, F&& f)
+
+// a / 9, correctly rounded (quotient's reasoning, below; for a result far
+// below the contrast's threshold, where an underflow could part them, both are 0).
+__device__ __forceinline__ float ninth(float a)
 {
-  const int bw = x1 - x0, gh = (y1 - y0 + VR - 1) / VR, n = bw * gh;
-  if (bw <= 0 || gh <= 0) return;
-  const int dq = VNT / bw, dr = VNT - dq * bw;
-  int q = (int)threadIdx.x / bw;
-  int c = (int)threadIdx.x - q * bw;
-  for (int i = threadIdx.x; i < n; i += VNT) {
-    const int ry = y0 + q * VR;
-    f(ry, x0 + c, min(VR, y1 - ry));
-    c += dr;
-    q += dq;
-    if (c >= bw) {
-      c -= bw;
-      ++q;
-    }
-  }
+  const float r = 1.0f / 9.0f, q = __fmul_rn(a, r);
+  return fmaf(fmaf(-9.0f, q, a), r, q);
 }
 
 __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
 
-// Gaussian (kind 3) or Sharpen (kind 4) with a K-tap kernel: the 1-D weights
-// in registers, a horizontal pass into `tmp`, then a vertical pass in column
-// units that reuse each loaded value for up to VR outputs.  Positions outside
-// the image hold 0 in every stage buffer, which is the reference's skipping
-// of out-of-image taps.
-template <bool IN, int K>
-__device__ void blur_stage(const FilterDev& f, const float* in, float* out, float* tmp, const Region& g, int lo, int hi)
+// k_view's dynamic shared memory, in 4-byte words: 4 words that a unit's
+// reads before a buffer's first row may touch, three stage buffers of P
+// columns, the VT x VT tile, then the region's per-column and per-row radiograph
+// mapping (texel index and weight each).  halo: the larger chain's.
+__host__ __device__ constexpr int view_ex(int halo) { return (halo + 3) & ~3; }
+__host__ __device__ constexpr int view_pitch(int halo) { return VT + 2 * view_ex(halo); }
+__host__ __device__ constexpr int view_rows(int halo) { return VT + 2 * halo; }
+__host__ __device__ constexpr size_t view_tail_floats(int halo)
 {
-  constexpr int R = K / 2;
-  const int E = g.E;
+  return 4 + (size_t)3 * view_rows(halo) * view_pitch(halo) + (size_t)VT * VT;
+}
+__host__ __device__ constexpr size_t view_smem_floats(int halo)
+{
+  return view_tail_floats(halo) + (size_t)2 * (view_rows(halo) + view_pitch(halo));
+}
+// the widest chain: three square stage buffers, the tile and ten words per
+// row of the region in 224 KB
+__host__ __device__ constexpr bool view_fits(int halo)
+{
+  const size_t E = view_rows(halo);
+  return (3 * E * E + (size_t)VT * VT + 10 * E) * 4 <= 224 * 1024;
+}
+static_assert(view_fits(42) && !view_fits(43) && view_smem_floats(42) * 4 + 2048 <= 227 * 1024,
+              "the widest chain fits a block's shared memory");
+constexpr int kNoTexel = -0x7fffffff;  // a column or row that maps outside the radiograph
+
+// Gaussian (kind 3) or Sharpen (kind 4) with a K-tap kernel: the 1-D weights
+// in registers, a horizontal pass into `tmp`, then a vertical pass, 4 columns
+// at a time in 16-byte words.  Each output adds its taps in order.  Positions
+// outside the image hold 0 in every stage buffer, which is the reference's
+// skipping of out-of-image taps.
+template <int K>
+__device__ void blur_stage(const FilterDev& f, const float* in, float* out, float* tmp, const Region& g, int halo)
+{
+  constexpr int R = K / 2, Q = (R + 3) / 4, NV = 2 * Q + 1;  // words on either side, words of a unit's reads
+  const int P = g.P;
   float w[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) w[k] = f.g[k];
-  for_band(lo - R, hi + R, lo, hi, [&](int ry, int rx) {
-    const float* p = in + ry * E + rx - R;
-    float sum = 0.f;
+  const Band b = band(g, halo);
+  for_units(Band{b.x0, b.x1, b.y0 - R, b.y1 + R}, [&](int ry, int rx) {
+    const float* p = in + ry * P + rx - 4 * Q;
+    float v[4 * NV];
 #pragma unroll
-    for (int k = 0; k < K; ++k) sum = fmaf(w[k], p[k], sum);
-    tmp[ry * E + rx] = sum;
+    for (int i = 0; i < NV; ++i) {
+      const float4 q = lds4(p + 4 * i);
+      v[4 * i] = q.x;
+      v[4 * i + 1] = q.y;
+      v[4 * i + 2] = q.z;
+      v[4 * i + 3] = q.w;
+    }
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = fmaf(w[k], v[4 * Q - R + i + k], s[i]);
+    *reinterpret_cast<float4*>(tmp + ry * P + rx) = make_float4(s[0], s[1], s[2], s[3]);
   });
   __syncthreads();
   const bool gauss = f.kind == 3;
   const float p1 = f.p1, p2 = f.p2;
-  for_units(lo, hi, lo, hi, [&](int ry, int rx, int nr) {
-    float col[K + VR - 1];
-    const float* p = tmp + (ry - R) * E + rx;
+  for_units(b, [&](int ry, int rx) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* p = tmp + (ry - R) * P + rx;
 #pragma unroll
-    for (int t = 0; t < K + VR - 1; ++t) col[t] = p[t * E];
+    for (int k = 0; k < K; ++k) {
+      const float4 q = lds4(p + k * P);
+      s[0] = fmaf(w[k], q.x, s[0]);
+      s[1] = fmaf(w[k], q.y, s[1]);
+      s[2] = fmaf(w[k], q.z, s[2]);
+      s[3] = fmaf(w[k], q.w, s[3]);
+    }
+    if (gauss) {
 #pragma unroll
-    for (int t = 0; t < VR; ++t) {
-      if (t < nr) {
-        float r = 0.f;
-        if (IN || inside(g, ry + t, rx)) {
-          float blur = 0.f;
+      for (int i = 0; i < 4; ++i) s[i] = clamp01(s[i]);
+    } else {
+      const float4 q = lds4(in + ry * P + rx);
 #pragma unroll
-          for (int k = 0; k < K; ++k) blur = fmaf(w[k], col[t + k], blur);
-          if (gauss) {
-            r = clamp01(blur);
-          } else {
-            const float v = in[(ry + t) * E + rx];
-            r = fabsf(v - blur) > p2 ? clamp01(v + p1 * (v - blur)) : v;
-          }
-        }
-        out[(ry + t) * E + rx] = r;
+      for (int i = 0; i < 4; ++i) {
+        const float v = part(q, i), blur = s[i];
+        s[i] = fabsf(v - blur) > p2 ? clamp01(v + p1 * (v - blur)) : v;
       }
     }
+    if (!g.in)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (!inside(g, ry, rx + i)) s[i] = 0.f;
+    *reinterpret_cast<float4*>(out + ry * P + rx) = make_float4(s[0], s[1], s[2], s[3]);
   });
 }
 
 // Any kernel size: per-element passes with the weights in shared memory.
-template <bool IN>
 __device__ void blur_stage_any(const FilterDev& f, const float* in, float* out, float* tmp, float* wsh,
-                               const Region& g, int lo, int hi)
+                               const Region& g, int halo)
 {
-  const int E = g.E, K = f.K, R = f.R;
+  const int P = g.P, K = f.K, R = f.R;
   const float p1 = f.p1, p2 = f.p2;
   if (threadIdx.x < K) wsh[threadIdx.x] = f.g[threadIdx.x];
   __syncthreads();
-  for_band(lo - R, hi + R, lo, hi, [&](int ry, int rx) {
-    const float* p = in + ry * E + rx - R;
+  const Band b = band(g, halo);
+  for_band(Band{b.x0, b.x1, b.y0 - R, b.y1 + R}, [&](int ry, int rx) {
+    const float* p = in + ry * P + rx - R;
     float sum = 0.f;
     for (int k = 0; k < K; ++k) sum = fmaf(wsh[k], p[k], sum);
-    tmp[ry * E + rx] = sum;
+    tmp[ry * P + rx] = sum;
   });
   __syncthreads();
-  for_band(lo, hi, lo, hi, [&](int ry, int rx) {
+  for_band(b, [&](int ry, int rx) {
     float r = 0.f;
-    if (IN || inside(g, ry, rx)) {
-      const float* p = tmp + (ry - R) * E + rx;
+    if (g.in || inside(g, ry, rx)) {
+      const float* p = tmp + (ry - R) * P + rx;
       float blur = 0.f;
-      for (int k = 0; k < K; ++k) blur = fmaf(wsh[k], p[k * E], blur);
+      for (int k = 0; k < K; ++k) blur = fmaf(wsh[k], p[k * P], blur);
       if (f.kind == 3) {
         r = clamp01(blur);
       } else {
-        const float v = in[ry * E + rx];
+        const float v = in[ry * P + rx];
         r = fabsf(v - blur) > p2 ? clamp01(v + p1 * (v - blur)) : v;
       }
     }
-    out[ry * E + rx] = r;
+    out[ry * P + rx] = r;
   });
 }
 
@@ -849,87 +892,102 @@ __device__ __forceinline__ float sobel_px(float p00, float p01, float p02, float
   return clamp01(s);
 }
 
-// Applies one filter from `in` to `out` over the square band
-// [lo, hi) x [lo, hi) of region coordinates; positions outside the image get
-// 0.  `tmp` holds the horizontal pass of a Gaussian/Sharpen blur, `wsh` the
-// 1-D weights of a blur of uncommon size.  IN: the region lies inside the
-// image.
-template <bool IN>
-__device__ void apply_stage(const FilterDev& f, const float* in, float* out, float* tmp, float* wsh, const Region& g,
-                            int lo, int hi)
+// The six columns rx - 1 .. rx + 4 of row p (p: column rx).
+__device__ __forceinline__ void six(const float* p, float* v)
 {
-  const int E = g.E;
+  const float4 c = lds4(p);
+  v[0] = p[-1];
+  v[1] = c.x;
+  v[2] = c.y;
+  v[3] = c.z;
+  v[4] = c.w;
+  v[5] = p[4];
+}
+
+// Applies one filter from `in` to `out` over the band of the tile and `halo`
+// pixels around it; positions outside the image get 0.  `tmp` holds the
+// horizontal pass of a Gaussian/Sharpen blur, `wsh` the 1-D weights of a blur
+// of uncommon size.
+__device__ void apply_stage(const FilterDev& f, const float* in, float* out, float* tmp, float* wsh, const Region& g,
+                            int halo)
+{
+  const int P = g.P;
   const int kind = f.kind, K = f.K;
   const float p0 = f.p0, p1 = f.p1;
   if (kind == 3 || kind == 4) {
     switch (K) {
-      case 3: blur_stage<IN, 3>(f, in, out, tmp, g, lo, hi); break;
-      case 5: blur_stage<IN, 5>(f, in, out, tmp, g, lo, hi); break;
-      case 7: blur_stage<IN, 7>(f, in, out, tmp, g, lo, hi); break;
-      case 9: blur_stage<IN, 9>(f, in, out, tmp, g, lo, hi); break;
-      case 11: blur_stage<IN, 11>(f, in, out, tmp, g, lo, hi); break;
-      case 13: blur_stage<IN, 13>(f, in, out, tmp, g, lo, hi); break;
-      default: blur_stage_any<IN>(f, in, out, tmp, wsh, g, lo, hi);
+      case 3: blur_stage<3>(f, in, out, tmp, g, halo); break;
+      case 5: blur_stage<5>(f, in, out, tmp, g, halo); break;
+      case 7: blur_stage<7>(f, in, out, tmp, g, halo); break;
+      case 9: blur_stage<9>(f, in, out, tmp, g, halo); break;
+      case 11: blur_stage<11>(f, in, out, tmp, g, halo); break;
+      case 13: blur_stage<13>(f, in, out, tmp, g, halo); break;
+      default: blur_stage_any(f, in, out, tmp, wsh, g, halo);
     }
   } else if (kind == 1) {
-    for_units(lo, hi, lo, hi, [&](int ry, int rx, int nr) {
-      float L[VR + 2], C[VR + 2], Rt[VR + 2];
-      const float* p = in + (ry - 1) * E + rx;
+    for_units(band(g, halo), [&](int ry, int rx) {
+      const float* p = in + ry * P + rx;
+      float u[6], m[6], d[6], o[4];
+      six(p - P, u);
+      six(p, m);
+      six(p + P, d);
 #pragma unroll
-      for (int t = 0; t < VR + 2; ++t) {
-        L[t] = p[t * E - 1];
-        C[t] = p[t * E];
-        Rt[t] = p[t * E + 1];
-      }
-#pragma unroll
-      for (int t = 0; t < VR; ++t) {
-        if (t < nr) {
+      for (int i = 0; i < 4; ++i)
+        o[i] = sobel_px(u[i], u[i + 1], u[i + 2], m[i], m[i + 1], m[i + 2], d[i], d[i + 1], d[i + 2], p0, p1);
+      if (!g.in)
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+          const int y = g.y0 + ry, x = g.x0 + rx + i;
+          if (x > 0 && x < g.w - 1 && y > 0 && y < g.h - 1) continue;
           float r = 0.f;
-          const int y = g.y0 + ry + t, x = g.x0 + rx;
-          if (IN || (x >= 0 && x < g.w && y >= 0 && y < g.h)) {
-            if (IN || (x > 0 && x < g.w - 1 && y > 0 && y < g.h - 1)) {
-              r = sobel_px(L[t], C[t], Rt[t], L[t + 1], C[t + 1], Rt[t + 1], L[t + 2], C[t + 2], Rt[t + 2], p0, p1);
-            } else {  // image border: neighbours outside the image repeat the edge
-              const int xm = x > 0 ? -1 : 0, xp = x < g.w - 1 ? 1 : 0, ym = y > 0 ? -E : 0, yp = y < g.h - 1 ? E : 0;
-              const float* c = in + (ry + t) * E + rx;
-              r = sobel_px(c[ym + xm], c[ym], c[ym + xp], c[xm], c[0], c[xp], c[yp + xm], c[yp], c[yp + xp], p0, p1);
-            }
+          if (x >= 0 && x < g.w && y >= 0 && y < g.h) {
+            // image border: neighbours outside the image repeat the edge
+            const int xm = x > 0 ? -1 : 0, xp = x < g.w - 1 ? 1 : 0, ym = y > 0 ? -P : 0, yp = y < g.h - 1 ? P : 0;
+            const float* c = p + i;
+            r = sobel_px(c[ym + xm], c[ym], c[ym + xp], c[xm], c[0], c[xp], c[yp + xm], c[yp], c[yp + xp], p0, p1);
           }
-          out[(ry + t) * E + rx] = r;
+          if (i == 0) o[0] = r;
+          if (i == 1) o[1] = r;
+          if (i == 2) o[2] = r;
+          if (i == 3) o[3] = r;
         }
-      }
+      *reinterpret_cast<float4*>(out + ry * P + rx) = make_float4(o[0], o[1], o[2], o[3]);
     });
   } else if (kind == 0 && K == 3) {
     // ContrastFilter_kernels.cu:62-96 with a 3 x 3 box: the mean over the
     // window's in-image pixels (out-of-image positions hold 0, so the sum
     // runs over the whole window and only the count depends on the border)
     const float e1 = p0 - p1, e2 = p1;
-    for_units(lo, hi, lo, hi, [&](int ry, int rx, int nr) {
-      float rs[VR + 2];
-      const float* p = in + (ry - 1) * E + rx - 1;
+    for_units(band(g, halo), [&](int ry, int rx) {
+      const float* p = in + ry * P + rx;
+      float u[6], m[6], d[6], o[4];
+      six(p - P, u);
+      six(p, m);
+      six(p + P, d);
 #pragma unroll
-      for (int t = 0; t < VR + 2; ++t) rs[t] = p[t * E] + p[t * E + 1] + p[t * E + 2];
+      for (int i = 0; i < 4; ++i)
+        o[i] = (u[i] + u[i + 1] + u[i + 2]) + (m[i] + m[i + 1] + m[i + 2]) + (d[i] + d[i + 1] + d[i + 2]);
 #pragma unroll
-      for (int t = 0; t < VR; ++t) {
-        if (t < nr) {
-          float r = 0.f;
-          const int y = g.y0 + ry + t, x = g.x0 + rx;
-          if (IN || (x >= 0 && x < g.w && y >= 0 && y < g.h)) {
-            float cnt = 9.0f;
-            if (!IN) cnt = (float)((min(y + 2, g.h) - max(y - 1, 0)) * (min(x + 2, g.w) - max(x - 1, 0)));
-            const float axy = (rs[t] + rs[t + 1] + rs[t + 2]) / cnt, v = in[(ry + t) * E + rx];
-            r = axy > 0.01f ? contrast_pow(axy, v, e1, e2) : 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        float axy = ninth(o[i]);
+        if (!g.in) {
+          const int y = g.y0 + ry, x = g.x0 + rx + i;
+          if (!(x > 0 && x < g.w - 1 && y > 0 && y < g.h - 1)) {
+            const bool at = x >= 0 && x < g.w && y >= 0 && y < g.h;
+            const int cnt = (min(y + 2, g.h) - max(y - 1, 0)) * (min(x + 2, g.w) - max(x - 1, 0));
+            axy = at ? o[i] / (float)cnt : 0.f;
           }
-          out[(ry + t) * E + rx] = r;
         }
+        o[i] = contrast_px(axy, m[i + 1], e1, e2);
       }
+      *reinterpret_cast<float4*>(out + ry * P + rx) = make_float4(o[0], o[1], o[2], o[3]);
     });
   } else if (kind == 0) {
     const int size = K, h0 = size / 2, h1 = (size + 1) / 2;
     const float e1 = p0 - p1, e2 = p1;
-    for_band(lo, hi, lo, hi, [&](int ry, int rx) {
+    for_band(band(g, halo), [&](int ry, int rx) {
       float r = 0.f;
-      if (IN || inside(g, ry, rx)) {
+      if (g.in || inside(g, ry, rx)) {
         const int x = g.x0 + rx, y = g.y0 + ry;
         const int i0 = max(y - h0, 0), i1 = min(y + h1, g.h);
         const int j0 = max(x - h0, 0), j1 = min(x + h1, g.w);
@@ -937,73 +995,157 @@ __device__ void apply_stage(const FilterDev& f, const float* in, float* out, flo
         for (int yy = i0; yy < i1; ++yy)
           for (int xx = j0; xx < j1; ++xx) {
             cnt += 1.0f;
-            sum += in[(yy - g.y0) * E + (xx - g.x0)];
+            sum += in[(yy - g.y0) * P + (xx - g.x0)];
           }
-        const float axy = sum / cnt, v = in[ry * E + rx];
+        const float axy = sum / cnt, v = in[ry * P + rx];
         r = axy > 0.01f ? contrast_pow(axy, v, e1, e2) : 0.0f;
       }
-      out[ry * E + rx] = r;
+      out[ry * P + rx] = r;
     });
   }
   __syncthreads();
 }
 
-// Runs a filter chain on buf[0] (valid on [eh - H, eh + VT + H)); returns the
-// buffer index holding the result on the tile band [eh, eh + VT).
-__device__ int run_chain(const FilterDev* fl, int nf, int H, float* bufs[3], float* wsh, const Region& g, int eh)
+// Runs a filter chain on the first of three stage buffers of `size` floats
+// each (valid on the tile and its halo H); returns the one holding the result on the tile.
+// Not inlined: both chains of a tile run the same code, which with it fits the instruction cache.
+__device__ __noinline__ float* run_chain(const FilterDev* fl, int nf, int H, float* buf, int size, float* wsh, Region g)
 {
-  int cur = 0, halo = H;
+  int halo = H;
+  float *in = buf, *out = buf + size;
   for (int s = 0; s < nf; ++s) {
-    const FilterDev& f = fl[s];
-    int nh = halo - f.R;
-    int nxt = cur == 0 ? 1 : 0;
-    if (g.in)
-      apply_stage<true>(f, bufs[cur], bufs[nxt], bufs[2], wsh, g, eh - nh, eh + VT + nh);
-    else
-      apply_stage<false>(f, bufs[cur], bufs[nxt], bufs[2], wsh, g, eh - nh, eh + VT + nh);
-    cur = nxt;
-    halo = nh;
+    halo -= fl[s].R;
+    apply_stage(fl[s], in, out, buf + 2 * size, wsh, g, halo);
+    float* t = in;
+    in = out;
+    out = t;
   }
-  return cur;
+  return in;
 }
 
+// The moments of a view's tiles, merged in FP64 by one warp: the exact mean
+// from the tiles' means, then each tile's co-moments moved to it (C + n
+// (mean - M)(mean' - M')), two sweeps with two divisions where merging the
+// tiles pairwise (Chan et al.) took eight levels of three.
+__device__ __forceinline__ double warp_sum_d(double v)
+{
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_WARP, v, o);
+  return v;
+}
+__device__ __forceinline__ Moments merge_tiles(const Moments* part, int nt)
+{
+  const int lane = threadIdx.x & 31;
+  Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int i = lane; i < nt; i += 32) {
+    const Moments* p = part + i;
+    const double n = __ldcg(&p->n);
+    a.sm += __ldcg(&p->sm);
+    a.sf += __ldcg(&p->sf);
+    a.sg += __ldcg(&p->sg);
+    a.n += n;
+    a.mf += n * __ldcg(&p->mf);
+    a.mg += n * __ldcg(&p->mg);
+  }
+  a.n = warp_sum_d(a.n);
+  a.sm = warp_sum_d(a.sm);
+  a.sf = warp_sum_d(a.sf);
+  a.sg = warp_sum_d(a.sg);
+  a.mf = warp_sum_d(a.mf);
+  a.mg = warp_sum_d(a.mg);
+  if (!(a.n > 0)) return a;
+  a.mf /= a.n;
+  a.mg /= a.n;
+  for (int i = lane; i < nt; i += 32) {
+    const Moments* p = part + i;
+    const double n = __ldcg(&p->n), df = __ldcg(&p->mf) - a.mf, dg = __ldcg(&p->mg) - a.mg;
+    if (n > 0) {
+      a.cff += __ldcg(&p->cff) + n * df * df;
+      a.cgg += __ldcg(&p->cgg) + n * dg * dg;
+      a.cfg += __ldcg(&p->cfg) + n * df * dg;
+    }
+  }
+  a.cff = warp_sum_d(a.cff);
+  a.cgg = warp_sum_d(a.cgg);
+  a.cfg = warp_sum_d(a.cfg);
+  return a;
+}
+
+// image_axis (asc_internal.cuh) with its two quotients by the crop's and the
+// image's fixed sizes taken from their reciprocals: q = RN(a r) corrected by
+// the exact remainder, q + r fma(-q, b, a), is the correctly rounded a / b
+// when r = RN(1 / b) (P. Markstein, IBM J. Res. Dev. 34(1), 1990), so the
+// result is the division's in 3 FP64 operations of a warp's ~70 cycles each.
+__device__ __forceinline__ double quotient(double a, double b, double r)
+{
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
+__device__ __forceinline__ bool view_axis(double v0, double vw, int x, int n, double rn, double i0, double iw, double riw,
+                                          int N, bool rows, int& k, float& a)
+{
+  const double u = v0 + vw * quotient((double)x, (double)n, rn);
+  const double q = quotient(u - i0, iw, riw);
+  const double s = rows ? 0.5 - q : q + 0.5;
+  if (s < 0.0 || s > 1.0) return false;
+  const double X = s * N - 0.5;
+  double fl = floor(X);
+  a = (float)(X - fl);
+  fl = fmin(fmax(fl, -1.0), (double)N);
+  k = (int)fl;
+  return true;
+}
+
+// One 48 x 48 output tile after another from a queue.  What bounds it is
+// instruction issue (55 %) and, at 24 warps per SM, the barriers between its
+// stages.  On 300 candidates x 2 views of 1024^2 with the four-filter chain:
+// 3.58 ms with one column per unit and the FP64 quotients by division, 2.84
+// here; 64 candidates under SAD at 771 x 645: 1.20 and 0.95.  The last
+// thread grabs the next tile while this one is filtered, and warp 0 alone
+// finishes a tile (its FP64 moments, the view's merge, the item's cost) while
+// the other warps go on to the next.
 __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     k_view(const SceneDev* __restrict__ sc, Bufs b, double* __restrict__ cost, double* __restrict__ view_cost_out)
 {
   extern __shared__ float smem[];
-  __shared__ int s_tile, s_k;
-  __shared__ bool s_last;
+  __shared__ int s_tile[2], s_k[2];  // this tile's and the next one's
   __shared__ float red[8 * 6 * 2];
   __shared__ double ds[6], dc[3];
+  __shared__ double s_rcp[4];  // 1 / w, 1 / h of the crop; 1 / the image's width and height on the film plane
   __shared__ float wsh[32];
-  Moments* msh = (Moments*)smem;          // reused by the merge
-  const int ns = sc->slots;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int tl = atomicAdd(&b.C->fnext, 1);
-      s_tile = tl;
-      s_k = tl < b.C->ftiles ? b.ftile_iv[tl] : 0;
+  __shared__ unsigned s_keep[VNT / 32];
+  const int ns = sc->slots, ftiles = b.C->ftiles;
+  const bool grabs = threadIdx.x == VNT - 1;
+  if (grabs) {
+    const int tl = atomicAdd(&b.C->fnext, 1);
+    s_tile[0] = tl;
+    s_k[0] = tl < ftiles ? b.ftile_iv[tl] : 0;
+  }
+  __syncthreads();
+  for (int turn = 0;; turn ^= 1) {
+    const int tile = s_tile[turn], k = s_k[turn];
+    if (tile >= ftiles) return;
+    int next = 0, next_k = 0;
+    if (grabs) {
+      next = atomicAdd(&b.C->fnext, 1);
+      next_k = next < ftiles ? b.ftile_iv[next] : 0;
     }
-    __syncthreads();
-    const int tile = s_tile, k = s_k;
-    __syncthreads();
-    if (tile >= b.C->ftiles) return;
     const IV& r = b.iv[k];
     const int t = tile - b.foff[k];
     const int tx0 = (t % r.ftx) * VT, ty0 = (t / r.ftx) * VT;
     const ViewDev& V = sc->views[r.view];
-    // this view's region edge E (its chain's halo) lays out the shared memory
-    const int E = V.E, eh = (E - VT) / 2;
-    float* bufs[3] = {smem, smem + E * E, smem + 2 * E * E};
-    float* fdrr = smem + 3 * E * E;  // VT x VT final DRR, then f = DRR * mask
+    // this view's halo lays out the shared memory
+    const int H = max(V.h_drr, V.h_rad), EX = view_ex(H), P = view_pitch(H), rows = view_rows(H);
+    const int size = rows * P;
+    float* buf = smem + 4;           // three stage buffers
+    float* fdrr = buf + 3 * size;  // VT x VT final DRR, then f = DRR * mask
     // per region column / row: the radiograph texel pair and weight of the
-    // film-plane mapping (image_axis; kNoTexel where the pixel maps outside)
-    int* tcx = (int*)(smem + view_tail_floats(E));
-    float* tax = (float*)(tcx + E);
-    int* tcy = (int*)(tax + E);
-    float* tay = (float*)(tcy + E);
-    const int rx0 = tx0 - eh, ry0 = ty0 - eh;
-    const Region g{rx0, ry0, E, r.w, r.h, rx0 >= 0 && ry0 >= 0 && rx0 + E <= r.w && ry0 + E <= r.h};
+    // film-plane mapping (view_axis; kNoTexel where the pixel maps outside)
+    int* tcx = (int*)(smem + view_tail_floats(H));
+    float* tax = (float*)(tcx + P);
+    int* tcy = (int*)(tax + P);
+    float* tay = (float*)(tcy + rows);
+    const int rx0 = tx0 - EX, ry0 = ty0 - H;
+    const Region g{rx0, ry0, P, EX, H, r.w, r.h, tx0 >= H && ry0 >= 0 && tx0 + VT + H <= r.w && ry0 + rows <= r.h};
     const float* drr = b.drr + r.pix;
     // ---- DRR region; a region of zeros filters to zeros (every filter maps
     // 0 to 0), so its tile masks out entirely and adds nothing to the moments
@@ -1011,63 +1153,87 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     {
       // the region's words copied asynchronously (all in flight at once;
       // zero-filled outside the image), then tested for a nonzero DRR
-      const int lo = eh - V.h_drr, hi = eh + VT + V.h_drr;
-      for_band(lo, hi, lo, hi, [&](int ry, int rx) {
+      const Band d = band(g, V.h_drr);
+      for_band(d, [&](int ry, int rx) {
         const bool in = g.in || inside(g, ry, rx);
         const float* src = in ? drr + (long long)(g.y0 + ry) * r.w + g.x0 + rx : drr;
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(bufs[0] + ry * E + rx);
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + ry * P + rx);
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 4 : 0)
                      : "memory");
       });
       asm volatile("cp.async.commit_group;\n" ::: "memory");
+      // meanwhile the reciprocals of the mapping's divisors
+      if (threadIdx.x < 4) {
+        const double v = threadIdx.x == 0 ? (double)r.w
+                                          : (threadIdx.x == 1 ? (double)r.h : (double)V.ipf[threadIdx.x == 2 ? 2 : 3]);
+        s_rcp[threadIdx.x] = 1.0 / v;
+      }
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       __syncthreads();
+      if (grabs) {  // for after this tile's last barrier
+        s_tile[turn ^ 1] = next;
+        s_k[turn ^ 1] = next_k;
+      }
       bool nz = false;
-      for_band(lo, hi, lo, hi, [&](int ry, int rx) { nz |= bufs[0][ry * E + rx] != 0.f; });
+      for_band(d, [&](int ry, int rx) { nz |= buf[ry * P + rx] != 0.f; });
       live = __syncthreads_or(nz);
     }
     float mf = 0.f, mg = 0.f;
     if (live) {
       // the film-plane mapping of the region's columns and rows, in FP64
       // (visible to the radiograph band after the chain's barriers)
-      for (int i = threadIdx.x; i < 2 * E; i += VNT) {
-        const bool row = i >= E;
-        const int j = row ? i - E : i;
-        int k;
+      for (int i = threadIdx.x; i < P + rows; i += VNT) {
+        const bool row = i >= P;
+        const int j = row ? i - P : i;
+        int q;
         float a = 0.f;
-        const bool ok = row ? image_axis(r.vp[1], r.vp[3], g.y0 + j, r.h, V.ipf[1], V.ipf[3], V.rad_h, true, k, a)
-                            : image_axis(r.vp[0], r.vp[2], g.x0 + j, r.w, V.ipf[0], V.ipf[2], V.rad_w, false, k, a);
-        (row ? tcy : tcx)[j] = ok ? k : kNoTexel;
+        const bool ok = row ? view_axis(r.vp[1], r.vp[3], g.y0 + j, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.rad_h,
+                                        true, q, a)
+                            : view_axis(r.vp[0], r.vp[2], g.x0 + j, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.rad_w,
+                                        false, q, a);
+        (row ? tcy : tcx)[j] = ok ? q : kNoTexel;
         (row ? tay : tax)[j] = a;
       }
       // ---- DRR chain
       {
-        int res = run_chain(V.fdrr, V.n_drr, V.h_drr, bufs, wsh, g, eh);
-        for (int i = threadIdx.x; i < VT * VT; i += VNT) fdrr[i] = bufs[res][(eh + i / VT) * E + eh + i % VT];
+        const float* res = run_chain(V.fdrr, V.n_drr, V.h_drr, buf, size, wsh, g) + H * P + EX;
+        for (int i = threadIdx.x; i < VT * VT / 4; i += VNT) {
+          const int ly = i / (VT / 4), lx = 4 * (i % (VT / 4));
+          *reinterpret_cast<float4*>(fdrr + ly * VT + lx) = lds4(res + ly * P + lx);
+        }
         __syncthreads();
       }
       // ---- radiograph crop and its chain
-      int rres;
+      float* gres;
       {
-        const int lo = eh - V.h_rad, hi = eh + VT + V.h_rad;
-        for_band(lo, hi, lo, hi, [&](int ry, int rx) {
+        for_band(band(g, V.h_rad), [&](int ry, int rx) {
           float val = 0.f;
           const int kx = tcx[rx], ky = tcy[ry];
           if ((g.in || inside(g, ry, rx)) && kx != kNoTexel && ky != kNoTexel)
             val = 1.0f - bilinear_at(V.rad, V.rad_bps, V.rad_w, V.rad_h, kx, tax[rx], ky, tay[ry]);
-          bufs[0][ry * E + rx] = val;
+          buf[ry * P + rx] = val;
         });
         __syncthreads();
-        rres = run_chain(V.frad, V.n_rad, V.h_rad, bufs, wsh, g, eh);
+        gres = run_chain(V.frad, V.n_rad, V.h_rad, buf, size, wsh, g) + H * P + EX;
       }
       // ---- masks and moments (Tracker.cpp:744-770), two passes over the
       // tile: f = DRR * mask over fdrr, g = rad * mask over the chain result,
       // the m > 0.5 flags in the free blur buffer
       const unsigned n = (unsigned)r.w * (unsigned)r.h;
       const bool tree = sc->coverage == ASC_SUM_TREE && tree_needed(n);  // else every pixel counts
+      // which pixels reach the reference's sum (tree_keep): every level but
+      // the last folds 256 partials and drops none, so it is the pixel's
+      // partial of the last level that counts, one bit of at most 256
+      int shift = 0;
+      if (tree) {
+        unsigned m = n;
+        for (; m > 256u; m = (m + 255u) >> 8) shift += 8;
+        const unsigned keep = __ballot_sync(FULL_WARP, threadIdx.x < m && tree_keep(threadIdx.x, m));
+        if ((threadIdx.x & 31) == 0) s_keep[threadIdx.x >> 5] = keep;
+        __syncthreads();
+      }
       const bool sad = sc->cf_model != 0;
-      float* gres = bufs[rres];
-      float* flag = bufs[2];
+      float* flag = buf + 2 * size;
       // per tile: the pixels with mask 1 and their sums of f and g.  The
       // mask is 0 or 1 and f, g are 0 where it is 0, so these are also the
       // covered pixels' sums of mask, f and g.  Plain FP32 suffices for them:
@@ -1076,16 +1242,17 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       float s[3] = {0.f, 0.f, 0.f};
       for (int i = threadIdx.x; i < VT * VT; i += VNT) {
         const int ly = i / VT, lx = i % VT, x = tx0 + lx, y = ty0 + ly;
-        const int gi = (eh + ly) * E + eh + lx;
+        const int gi = ly * P + lx;
         float f = 0.f, gm = 0.f, fl = 0.f;
-        if (x < r.w && y < r.h && (!tree || tree_keep((unsigned)(y * r.w + x), n))) {
+        const unsigned at = (unsigned)(y * r.w + x) >> shift;
+        if (x < r.w && y < r.h && (!tree || (s_keep[at >> 5] >> (at & 31u) & 1u))) {
           float d = fdrr[i], gg = gres[gi];
           float bg = 1.0f;
           if (V.bg && V.bg_thr >= 0.f) {
             int kx, ky;
             float ax, ay;
-            bg = image_axis(r.vp[0], r.vp[2], x, r.w, V.ipf[0], V.ipf[2], V.bg_w, false, kx, ax) &&
-                     image_axis(r.vp[1], r.vp[3], y, r.h, V.ipf[1], V.ipf[3], V.bg_h, true, ky, ay)
+            bg = view_axis(r.vp[0], r.vp[2], x, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.bg_w, false, kx, ax) &&
+                     view_axis(r.vp[1], r.vp[3], y, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.bg_h, true, ky, ay)
                    ? (V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, ax, ky, ay) ? 1.0f : 0.0f)
                    : 0.0f;
           }
@@ -1105,63 +1272,58 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         // SAD needs the view's global means first: keep f and g for k_sad
         if (sad && x < r.w && y < r.h) b.fg[r.pix + (long long)y * r.w + x] = make_float2(f, gm);
       }
+      // the sums (ds[3 ..]), and the tile's FP32 centres from them
       block_sum_f<3>(s, red, ds + 3);
-      if (threadIdx.x < 3) ds[threadIdx.x] = ds[3 + threadIdx.x];  // read by thread 0 after the next barrier
-      const double cnt = ds[3];
-      mf = cnt > 0 ? (float)(ds[4] / cnt) : 0.f;
-      mg = cnt > 0 ? (float)(ds[5] / cnt) : 0.f;
+      if (threadIdx.x < 3) {
+        const double cnt = ds[3], mine = ds[3 + threadIdx.x];
+        ds[threadIdx.x] = mine;
+        red[threadIdx.x] = cnt > 0 ? (float)(mine / cnt) : 0.f;
+      }
+      __syncthreads();
+      mf = red[1];
+      mg = red[2];
       DFs c[3] = {};  // compensated co-moments about (mf, mg)
       for (int i = threadIdx.x; i < VT * VT && !sad; i += VNT)
         if (flag[i] != 0.f) {
           const int ly = i / VT, lx = i % VT;
-          float a = fdrr[i] - mf, bb = gres[(eh + ly) * E + eh + lx] - mg;
+          float a = fdrr[i] - mf, bb = gres[ly * P + lx] - mg;
           dfs_add_prod(c[0], a, a);
           dfs_add_prod(c[1], bb, bb);
           dfs_add_prod(c[2], a, bb);
         }
       block_sum_dfs<3>(c, red, dc);
-    } else if (threadIdx.x == 0) {  // a tile of zeros adds nothing
-      for (int j = 0; j < 6; ++j) ds[j] = 0.0;
-      for (int j = 0; j < 3; ++j) dc[j] = 0.0;
     }
-    if (threadIdx.x == 0) {
-      Moments p = tile_moments(ds, dc, mf, mg);
-      b.part[tile] = p;
+    if (threadIdx.x >= 32) continue;
+    // ---- warp 0: the tile's moments; the last tile of a view merges its
+    // tiles, the last view of an item sums the view costs
+    const int lane = threadIdx.x, nt = r.ftx * r.fty;
+    bool last = false;
+    if (lane == 0) {
+      const double zero[6] = {0, 0, 0, 0, 0, 0};
+      b.part[tile] = live ? tile_moments(ds, dc, mf, mg) : tile_moments(zero, zero, 0.f, 0.f);  // zeros add nothing
       __threadfence();
-      s_last = atomicAdd(&b.ivt[k], 1u) == (unsigned)(r.ftx * r.fty) - 1;
+      last = atomicAdd(&b.ivt[k], 1u) == (unsigned)nt - 1;
     }
-    __syncthreads();
-    if (!s_last) continue;
+    if (!__shfl_sync(FULL_WARP, (int)last, 0)) continue;
     __threadfence();
-    // ---- last tile of this view: merge its tiles in FP64
-    const int nt = r.ftx * r.fty, base = b.foff[k];
-    Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) moments_merge(a, b.part[base + i]);
-    msh[threadIdx.x] = a;
-    __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-      if (threadIdx.x < st) moments_merge(msh[threadIdx.x], msh[threadIdx.x + st]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0 && sc->cf_model) {
+    const Moments m = merge_tiles(b.part + b.foff[k], nt);
+    if (lane != 0) continue;
+    if (sc->cf_model) {
       // HDist_kernels.cu:111-115: the means over the mask sum; k_sad takes
       // the view from here and reuses its tile tickets
-      const Moments& m = msh[0];
       b.hmean[k] = make_double2(m.sf / m.sm, m.sg / m.sm);
       b.ivt[k] = 0;
-    } else if (threadIdx.x == 0) {
-      double vc = 1.0 - moments_ncc(msh[0]);
-      b.vcost[k] = vc;
-      __threadfence();
-      const int item = k / ns;
-      if (atomicAdd(&b.itt[item], 1u) == (unsigned)ns - 1) {
-        __threadfence();
-        finish_item(sc, b, item, cost);
-        if (view_cost_out)
-          for (int j = 0; j < ns; ++j) view_cost_out[item * ns + j] = b.vcost[item * ns + j];
-      }
+      continue;
     }
-    __syncthreads();
+    b.vcost[k] = 1.0 - moments_ncc(m);
+    __threadfence();
+    const int item = k / ns;
+    if (atomicAdd(&b.itt[item], 1u) == (unsigned)ns - 1) {
+      __threadfence();
+      finish_item(sc, b, item, cost);
+      if (view_cost_out)
+        for (int j = 0; j < ns; ++j) view_cost_out[item * ns + j] = b.vcost[item * ns + j];
+    }
   }
 }
 
@@ -1472,10 +1634,7 @@ static int fill_view(ViewDev& d, const asc_view_desc& v)
   n = prep_filters(v.rad_filters, v.n_rad_filters, d.frad, &d.h_rad);
   if (n < 0) return n;
   d.n_rad = n;
-  d.E = VT + 2 * std::max(d.h_drr, d.h_rad);
-  // three E x E stage buffers, the tile and the mapping tables must fit one
-  // block's shared memory (227 KB less the static arrays)
-  if (view_smem_floats(d.E) * sizeof(float) > 224 * 1024) return ASC_ERR_RANGE;
+  if (!view_fits(std::max(d.h_drr, d.h_rad))) return ASC_ERR_RANGE;
   return ASC_OK;
 }
 
@@ -1531,7 +1690,7 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
   S.coverage = coverage;
   S.cf_model = cf_model;
   S.slots = std::min(n_views, MAX_SLOTS);
-  S.E = 0;
+  S.halo = 0;
   for (int v = 0; v < n_views; ++v) {
     int rc = fill_view(S.views[v], views[v]);
     if (rc) {
@@ -1540,7 +1699,7 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
     }
     S.views[v].rw = rw;
     S.views[v].rh = rh;
-    S.E = std::max(S.E, S.views[v].E);
+    S.halo = std::max({S.halo, S.views[v].h_drr, S.views[v].h_rad});
   }
   for (int i = 0; i < n_bones; ++i) {
     auto* vh = (asc_volume_host*)bones[i].volume;
@@ -1622,10 +1781,7 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
     delete e;
     return ASC_ERR_CUDA;
   }
-  // three stage buffers, the final DRR tile and VR + 2 rows of slack for the
-  // column units' reads past a band
-  e->smem = view_smem_floats(S.E) * sizeof(float);
-  e->smem = std::max(e->smem, (size_t)256 * sizeof(Moments));
+  e->smem = view_smem_floats(S.halo) * sizeof(float);
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1695,14 +1851,15 @@ ASC_API int asc_engine_set_view(asc_engine e, int view, const asc_view_desc* des
   d.rw = rw;
   d.rh = rh;
   Gate g(device_gate());
-  const size_t need = view_smem_floats(d.E) * sizeof(float);
+  const int halo = std::max(d.h_drr, d.h_rad);
+  const size_t need = view_smem_floats(halo) * sizeof(float);
   if (need > e->smem) {  // a wider filter chain than the engine's views had so far
     int blocks = 0;
     ASC_CUDA(ensure_view_smem(need));
     ASC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_view, VNT, need));
     e->smem = need;
     e->view_blocks = std::max(blocks, 1);
-    e->host.E = std::max(e->host.E, d.E);
+    e->host.halo = std::max(e->host.halo, halo);
     if (e->pso_exec) {  // its k_view node holds the old launch shape
       cudaGraphExecDestroy(e->pso_exec);
       e->pso_exec = nullptr;

@@ -583,7 +583,7 @@ __device__ __forceinline__ RayScene ray_scene(const IV& r, const BoneDev& B, int
 __global__ void __launch_bounds__(NRAY, ASC_RAY_MINBLOCKS) k_ray(const SceneDev* __restrict__ sc, Bufs b, int skip,
                                                                  int shape)
 {
-  __shared__ RaySlots S;
+  __shared__ RaySlots<NRAY> S;
   const int lane = threadIdx.x & 31;
   const unsigned n = (unsigned)b.C->rtiles * BEAMS;
   unsigned long long marched = 0, slots = 0;
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(NRAY, ASC_RAY_MINBLOCKS) k_ray(const SceneDev*
       continue;
     }
     unsigned done = 0, room = 0;
-    const float d = ray_beam(B.vol, s, B.cut[r.slot], make_float4(r.band[0], r.band[1], r.band[2], 0.f), S, x, y, valid,
+    const float d = ray_beam<1>(B.vol, s, B.cut[r.slot], make_float4(r.band[0], r.band[1], r.band[2], 0.f), S, x, y, valid,
                              beam, done, room);
     marched += done;
     slots += room;
@@ -745,14 +745,6 @@ __device__ __forceinline__ float contrast_pow(float axy, float v, float e1, floa
 __device__ __forceinline__ float contrast_px(float axy, float v, float e1, float e2)
 {
   return axy > 0.01f ? contrast_pow(axy, v, e1, e2) : 0.0f;
-}
-
-// a / 9, correctly rounded (quotient's reasoning, below; for a result far
-// below the contrast's threshold, where an underflow could part them, both are 0).
-__device__ __forceinline__ float ninth(float a)
-{
-  const float r = 1.0f / 9.0f, q = __fmul_rn(a, r);
-  return fmaf(fmaf(-9.0f, q, a), r, q);
 }
 
 __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
@@ -1023,78 +1015,6 @@ __device__ __noinline__ float* run_chain(const FilterDev* fl, int nf, int H, flo
   return in;
 }
 
-// The moments of a view's tiles, merged in FP64 by one warp: the exact mean
-// from the tiles' means, then each tile's co-moments moved to it (C + n
-// (mean - M)(mean' - M')), two sweeps with two divisions where merging the
-// tiles pairwise (Chan et al.) took eight levels of three.
-__device__ __forceinline__ double warp_sum_d(double v)
-{
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_WARP, v, o);
-  return v;
-}
-__device__ __forceinline__ Moments merge_tiles(const Moments* part, int nt)
-{
-  const int lane = threadIdx.x & 31;
-  Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = lane; i < nt; i += 32) {
-    const Moments* p = part + i;
-    const double n = __ldcg(&p->n);
-    a.sm += __ldcg(&p->sm);
-    a.sf += __ldcg(&p->sf);
-    a.sg += __ldcg(&p->sg);
-    a.n += n;
-    a.mf += n * __ldcg(&p->mf);
-    a.mg += n * __ldcg(&p->mg);
-  }
-  a.n = warp_sum_d(a.n);
-  a.sm = warp_sum_d(a.sm);
-  a.sf = warp_sum_d(a.sf);
-  a.sg = warp_sum_d(a.sg);
-  a.mf = warp_sum_d(a.mf);
-  a.mg = warp_sum_d(a.mg);
-  if (!(a.n > 0)) return a;
-  a.mf /= a.n;
-  a.mg /= a.n;
-  for (int i = lane; i < nt; i += 32) {
-    const Moments* p = part + i;
-    const double n = __ldcg(&p->n), df = __ldcg(&p->mf) - a.mf, dg = __ldcg(&p->mg) - a.mg;
-    if (n > 0) {
-      a.cff += __ldcg(&p->cff) + n * df * df;
-      a.cgg += __ldcg(&p->cgg) + n * dg * dg;
-      a.cfg += __ldcg(&p->cfg) + n * df * dg;
-    }
-  }
-  a.cff = warp_sum_d(a.cff);
-  a.cgg = warp_sum_d(a.cgg);
-  a.cfg = warp_sum_d(a.cfg);
-  return a;
-}
-
-// image_axis (asc_internal.cuh) with its two quotients by the crop's and the
-// image's fixed sizes taken from their reciprocals: q = RN(a r) corrected by
-// the exact remainder, q + r fma(-q, b, a), is the correctly rounded a / b
-// when r = RN(1 / b) (P. Markstein, IBM J. Res. Dev. 34(1), 1990), so the
-// result is the division's in 3 FP64 operations of a warp's ~70 cycles each.
-__device__ __forceinline__ double quotient(double a, double b, double r)
-{
-  const double q = a * r;
-  return fma(fma(-q, b, a), r, q);
-}
-__device__ __forceinline__ bool view_axis(double v0, double vw, int x, int n, double rn, double i0, double iw, double riw,
-                                          int N, bool rows, int& k, float& a)
-{
-  const double u = v0 + vw * quotient((double)x, (double)n, rn);
-  const double q = quotient(u - i0, iw, riw);
-  const double s = rows ? 0.5 - q : q + 0.5;
-  if (s < 0.0 || s > 1.0) return false;
-  const double X = s * N - 0.5;
-  double fl = floor(X);
-  a = (float)(X - fl);
-  fl = fmin(fmax(fl, -1.0), (double)N);
-  k = (int)fl;
-  return true;
-}
-
 // One 48 x 48 output tile after another from a queue.  What bounds it is
 // instruction issue (55 %) and, at 24 warps per SM, the barriers between its
 // stages.  On 300 candidates x 2 views of 1024^2 with the four-filter chain:
@@ -1139,7 +1059,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     float* buf = smem + 4;           // three stage buffers
     float* fdrr = buf + 3 * size;  // VT x VT final DRR, then f = DRR * mask
     // per region column / row: the radiograph texel pair and weight of the
-    // film-plane mapping (view_axis; kNoTexel where the pixel maps outside)
+    // film-plane mapping (image_axis; kNoTexel where the pixel maps outside)
     int* tcx = (int*)(smem + view_tail_floats(H));
     float* tax = (float*)(tcx + P);
     int* tcy = (int*)(tax + P);
@@ -1166,7 +1086,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       if (threadIdx.x < 4) {
         const double v = threadIdx.x == 0 ? (double)r.w
                                           : (threadIdx.x == 1 ? (double)r.h : (double)V.ipf[threadIdx.x == 2 ? 2 : 3]);
-        s_rcp[threadIdx.x] = 1.0 / v;
+        s_rcp[threadIdx.x] = reciprocal(v);
       }
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       __syncthreads();
@@ -1187,10 +1107,10 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         const int j = row ? i - P : i;
         int q;
         float a = 0.f;
-        const bool ok = row ? view_axis(r.vp[1], r.vp[3], g.y0 + j, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.rad_h,
-                                        true, q, a)
-                            : view_axis(r.vp[0], r.vp[2], g.x0 + j, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.rad_w,
-                                        false, q, a);
+        const bool ok = row ? image_axis(r.vp[1], r.vp[3], g.y0 + j, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.rad_h,
+                                         true, q, a)
+                            : image_axis(r.vp[0], r.vp[2], g.x0 + j, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.rad_w,
+                                         false, q, a);
         (row ? tcy : tcx)[j] = ok ? q : kNoTexel;
         (row ? tay : tax)[j] = a;
       }
@@ -1221,15 +1141,9 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       // the m > 0.5 flags in the free blur buffer
       const unsigned n = (unsigned)r.w * (unsigned)r.h;
       const bool tree = sc->coverage == ASC_SUM_TREE && tree_needed(n);  // else every pixel counts
-      // which pixels reach the reference's sum (tree_keep): every level but
-      // the last folds 256 partials and drops none, so it is the pixel's
-      // partial of the last level that counts, one bit of at most 256
       int shift = 0;
       if (tree) {
-        unsigned m = n;
-        for (; m > 256u; m = (m + 255u) >> 8) shift += 8;
-        const unsigned keep = __ballot_sync(FULL_WARP, threadIdx.x < m && tree_keep(threadIdx.x, m));
-        if ((threadIdx.x & 31) == 0) s_keep[threadIdx.x >> 5] = keep;
+        shift = tree_mask(n, s_keep);
         __syncthreads();
       }
       const bool sad = sc->cf_model != 0;
@@ -1244,15 +1158,14 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         const int ly = i / VT, lx = i % VT, x = tx0 + lx, y = ty0 + ly;
         const int gi = ly * P + lx;
         float f = 0.f, gm = 0.f, fl = 0.f;
-        const unsigned at = (unsigned)(y * r.w + x) >> shift;
-        if (x < r.w && y < r.h && (!tree || (s_keep[at >> 5] >> (at & 31u) & 1u))) {
+        if (x < r.w && y < r.h && (!tree || tree_kept(s_keep, (unsigned)(y * r.w + x), shift))) {
           float d = fdrr[i], gg = gres[gi];
           float bg = 1.0f;
           if (V.bg && V.bg_thr >= 0.f) {
             int kx, ky;
             float ax, ay;
-            bg = view_axis(r.vp[0], r.vp[2], x, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.bg_w, false, kx, ax) &&
-                     view_axis(r.vp[1], r.vp[3], y, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.bg_h, true, ky, ay)
+            bg = image_axis(r.vp[0], r.vp[2], x, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.bg_w, false, kx, ax) &&
+                     image_axis(r.vp[1], r.vp[3], y, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.bg_h, true, ky, ay)
                    ? (V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, ax, ky, ay) ? 1.0f : 0.0f)
                    : 0.0f;
           }
@@ -1306,7 +1219,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     }
     if (!__shfl_sync(FULL_WARP, (int)last, 0)) continue;
     __threadfence();
-    const Moments m = merge_tiles(b.part + b.foff[k], nt);
+    const Moments m = merge_moments(b.part + b.foff[k], nt);
     if (lane != 0) continue;
     if (sc->cf_model) {
       // HDist_kernels.cu:111-115: the means over the mask sum; k_sad takes
@@ -1547,7 +1460,7 @@ struct asc_engine_s {
   // plain per-pose path: the reference's Tracker buffers (Tracker.cpp:292-298)
   std::vector<asc_view_desc> vdesc;
   std::vector<asc_bone_desc> bdesc;
-  float *p_drr = nullptr, *p_rad = nullptr, *p_mask = nullptr, *p_bg = nullptr, *p_tmp = nullptr, *p_bgr = nullptr;
+  float *p_drr = nullptr, *p_rad = nullptr, *p_mask = nullptr, *p_tmp = nullptr, *p_bgr = nullptr;
   double* p_res = nullptr;
   std::vector<void*> allocs;
   // clearance grids of bones replaced by asc_engine_set_bone, per (bone,
@@ -1765,7 +1678,6 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
   if (!err) err = e->alloc(e->p_drr, npix);
   if (!err) err = e->alloc(e->p_rad, npix);
   if (!err) err = e->alloc(e->p_mask, npix);
-  if (!err) err = e->alloc(e->p_bg, npix);
   if (!err) err = e->alloc(e->p_tmp, npix);
   if (!err) err = e->alloc(e->p_bgr, npix);
   if (!err) err = e->alloc(e->p_res, 1);
@@ -1777,7 +1689,7 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
   }
   e->vdesc.assign(views, views + n_views);
   e->bdesc.assign(bones, bones + n_bones);
-  if (asc_fill(e->p_bg, npix, 1.0f, cs) || cudaStreamSynchronize(cs)) {
+  if (cudaStreamSynchronize(cs)) {
     delete e;
     return ASC_ERR_CUDA;
   }
@@ -2292,7 +2204,7 @@ static int render_bone(const BoneDev& B, const asc_bone_desc& BD, int v, const f
     return ASC_OK;
   }
   return raycast_launch(B.vol, g_empty_skip ? B.clr[v] : nullptr, m, vpf, BD.step[v], BD.intensity[v], BD.cutoff[v],
-                        out, w, h, s);
+                        out, false, w, h, s);
 }
 
 ASC_API int asc_engine_eval_plain(asc_engine e, int n, const int* bone, const double* manip, double* cost,
@@ -2346,15 +2258,12 @@ ASC_API int asc_engine_eval_plain(asc_engine e, int n, const int* bone, const do
           float *r = e->p_rad, *ro = o;
           if (!rc) rc = chain_plain(VD.rad_filters, VD.n_rad_filters, r, ro, w, h, s);
           float* mask = e->p_mask;
-          float* bgm = e->p_bg;  // all ones: the mask of a disabled background
+          float* bgm = nullptr;  // no background: a mask of ones
           if (!rc && VD.background && VD.bg_threshold >= 0) {
             bgm = e->p_bgr;
             rc = asc_background_render(VD.background, V.ipf, vpf, VD.bg_threshold, bgm, w, h, s);
           }
-          if (!rc) rc = asc_drr_background(d, mask, w, h, s);
-          if (!rc) rc = asc_multiply(bgm, mask, mask, w, h, s);
-          if (!rc) rc = asc_multiply(r, mask, r, w, h, s);
-          if (!rc) rc = asc_multiply(d, mask, d, w, h, s);
+          if (!rc) rc = mask_images(d, r, bgm, mask, d, r, (size_t)w * h, s);
           double res = 0;
           if (!rc)
             rc = S_.cf_model ? asc_hdist(d, r, mask, w * h, S_.coverage, e->p_res, s)
@@ -2620,8 +2529,8 @@ ASC_API int asc_engine_render_drr(asc_engine e, int view, const double* poses, c
   if (w == 0 || h == 0) return ASC_OK;
   const float vpf[4] = {(float)vp[0], (float)vp[1], (float)vp[2], (float)vp[3]};
   // View::renderDrr (View.cpp:201-231): each bone's DRR merged (sum clamped
-  // to 1) into a zeroed buffer, then the view's DRR filters
-  ASC_CUDA(cudaMemsetAsync(e->p_mask, 0, (size_t)w * h * sizeof(float), s));
+  // to 1) into a zeroed buffer, then the view's DRR filters.  The first DRR is the merge with zeros
+  bool any = false;
   for (int b = 0; b < e->n_bones; ++b) {
     const BoneDev& B = e->host.bones[b];
     const asc_bone_desc& BD = e->bdesc[b];
@@ -2629,10 +2538,11 @@ ASC_API int asc_engine_render_drr(asc_engine e, int view, const double* poses, c
     view_matrix(V, B, poses + 6 * b, m);
     if (!B.visible) continue;  // its zeros leave the merge unchanged
     int rc = raycast_launch(B.vol, g_empty_skip ? B.clr[view] : nullptr, m, vpf, BD.step[view], BD.intensity[view],
-                            BD.cutoff[view], e->p_drr, w, h, s);
-    if (!rc) rc = asc_merge(e->p_mask, e->p_drr, e->p_mask, w, h, s);
+                            BD.cutoff[view], e->p_mask, any, w, h, s);
     if (rc) return rc;
+    any = true;
   }
+  if (!any) ASC_CUDA(cudaMemsetAsync(e->p_mask, 0, (size_t)w * h * sizeof(float), s));
   float *d = e->p_mask, *o = e->p_tmp;
   int rc = chain_plain(VD.drr_filters, VD.n_drr_filters, d, o, w, h, s);
   if (!rc) ASC_CUDA(cudaMemcpyAsync(out, d, (size_t)w * h * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -2663,15 +2573,12 @@ ASC_API int asc_engine_image_data(asc_engine e, int view, int bone, const double
   if (!rc) rc = asc_rad_render(VD.radiograph, V.ipf, vpf, e->p_rad, w, h, s);
   float *r = e->p_rad, *ro = o;
   if (!rc) rc = chain_plain(VD.rad_filters, VD.n_rad_filters, r, ro, w, h, s);
-  float* bgm = e->p_bg;
+  float* bgm = nullptr;
   if (!rc && VD.background && VD.bg_threshold >= 0) {
     bgm = e->p_bgr;
     rc = asc_background_render(VD.background, V.ipf, vpf, VD.bg_threshold, bgm, w, h, s);
   }
-  if (!rc) rc = asc_drr_background(d, mask, w, h, s);
-  if (!rc) rc = asc_multiply(bgm, mask, mask, w, h, s);
-  if (!rc) rc = asc_multiply(r, mask, rad, w, h, s);
-  if (!rc) rc = asc_multiply(d, mask, drr, w, h, s);
+  if (!rc) rc = mask_images(d, r, bgm, mask, drr, rad, (size_t)w * h, s);
   if (rc) return rc;
   if (width) *width = w;
   if (height) *height = h;

@@ -90,11 +90,33 @@ __device__ __forceinline__ float image_texel(const void* img, int bps, int i)
 // FP64 mapping leaves only the FP32 interpolation's rounding.  Every pixel
 // of a column (row) shares its column's (row's) mapping, so a tile computes
 // it once per column and once per row.
-__host__ __device__ __forceinline__ bool image_axis(double v0, double vw, int x, int n, double i0, double iw, int N,
-                                                    bool rows, int& k, float& a)
+//
+// The two quotients, by n and iw, take those divisors' reciprocals rn and
+// riw (correctly rounded): q = RN(a r) corrected by its exact remainder, q +
+// r fma(-q, b, a), is the correctly rounded a / b (P. Markstein, IBM J. Res.
+// Dev. 34(1), 1990; here b has at most 32 bits, so no quotient lies within 2^-33 ulp of a rounding
+// boundary, while the correction errs by less than 2^-50), at three FP64 operations
+// instead of a division's.
+// A divisor without a finite reciprocal (reciprocal() is then 0) and quotients
+// that are not finite take the division's own result.
+__host__ __device__ __forceinline__ double reciprocal(double b) { return b == 0.0 ? 0.0 : 1.0 / b; }
+__host__ __device__ __noinline__ inline double divided(double a, double b) { return a / b; }
+__host__ __device__ __forceinline__ double quotient(double a, double b, double r)
 {
-  const double u = v0 + vw * ((double)x / (double)n);
-  const double q = (u - i0) / iw;
+  const double q = a * r;
+#ifdef __CUDA_ARCH__
+  // on the high words: an FP64 comparison would cost what a step of the correction does
+  if (__double2hiint(r) == 0 || (__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return divided(a, b);
+#else
+  if (r == 0.0 || !(q - q == 0.0)) return divided(a, b);
+#endif
+  return fma(fma(-q, b, a), r, q);
+}
+__host__ __device__ __forceinline__ bool image_axis(double v0, double vw, int x, int n, double rn, double i0, double iw,
+                                                    double riw, int N, bool rows, int& k, float& a)
+{
+  const double u = v0 + vw * quotient((double)x, (double)n, rn);
+  const double q = quotient(u - i0, iw, riw);
   const double s = rows ? 0.5 - q : q + 0.5;
   if (s < 0.0 || s > 1.0) return false;
   const double X = s * N - 0.5;
@@ -103,6 +125,14 @@ __host__ __device__ __forceinline__ bool image_axis(double v0, double vw, int x,
   fl = fmin(fmax(fl, -1.0), (double)N);
   k = (int)fl;
   return true;
+}
+
+// a / 9, correctly rounded, by the same correction (a result so small that an
+// underflow could part them is 0 to the contrast filter either way).
+__device__ __forceinline__ float ninth(float a)
+{
+  const float r = 1.0f / 9.0f, q = __fmul_rn(a, r);
+  return fmaf(fmaf(-9.0f, q, a), r, q);
 }
 
 // Bilinear read of an 8/16-bit (normalized) or float image at the pair
@@ -152,9 +182,26 @@ __host__ __device__ __forceinline__ bool tree_keep(unsigned i, unsigned n)
   return true;
 }
 
-// Moments of one block or tile for the NCC (combined in FP64 with Chan et
-// al.'s pairwise update): sums over all covered pixels, and count, means and
-// co-moments over the covered pixels whose mask > 0.5.
+// tree_keep for many elements: every level but the last folds 256 partials
+// and drops none, so it is the element's partial of the last level that
+// counts, one bit of at most 256.  A block of 256 threads fills s_keep (8
+// words; a barrier before it is read) and returns the levels' shift.
+__device__ __forceinline__ int tree_mask(unsigned n, unsigned* s_keep)
+{
+  int shift = 0;
+  for (; n > 256u; n = (n + 255u) >> 8) shift += 8;
+  const unsigned keep = __ballot_sync(0xffffffffu, threadIdx.x < n && tree_keep(threadIdx.x, n));
+  if ((threadIdx.x & 31) == 0) s_keep[threadIdx.x >> 5] = keep;
+  return shift;
+}
+__device__ __forceinline__ bool tree_kept(const unsigned* s_keep, unsigned i, int shift)
+{
+  const unsigned at = i >> shift;
+  return s_keep[at >> 5] >> (at & 31u) & 1u;
+}
+
+// Moments of one block or tile for the NCC: sums over all covered pixels, and
+// count, means and co-moments over the covered pixels whose mask > 0.5.
 struct Moments {
   double sm, sf, sg;   // sum of mask, f, g over covered pixels
   double n;            // covered pixels with mask > 0.5
@@ -162,24 +209,51 @@ struct Moments {
   double cff, cgg, cfg;  // their centred co-moments
 };
 
-__host__ __device__ inline void moments_merge(Moments& a, const Moments& b)
+// The moments of `nb` blocks or tiles, merged in FP64 by one warp: the exact
+// mean from theirs, then each one's co-moments moved to it (C + n (mean - M)
+// (mean' - M')), two sweeps with two divisions where merging them pairwise
+// (Chan et al.) took eight levels of three, at ~70 cycles an operation.
+__device__ __forceinline__ double warp_sum_d(double v)
 {
-  a.sm += b.sm;
-  a.sf += b.sf;
-  a.sg += b.sg;
-  double n = a.n + b.n;
-  if (b.n == 0) return;
-  if (a.n == 0) {
-    a.n = b.n; a.mf = b.mf; a.mg = b.mg; a.cff = b.cff; a.cgg = b.cgg; a.cfg = b.cfg;
-    return;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
+{
+  const int lane = threadIdx.x & 31;
+  Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int i = lane; i < nb; i += 32) {
+    const Moments* p = part + i;
+    const double n = __ldcg(&p->n);
+    a.sm += __ldcg(&p->sm);
+    a.sf += __ldcg(&p->sf);
+    a.sg += __ldcg(&p->sg);
+    a.n += n;
+    a.mf += n * __ldcg(&p->mf);
+    a.mg += n * __ldcg(&p->mg);
   }
-  double df = b.mf - a.mf, dg = b.mg - a.mg, k = a.n * b.n / n;
-  a.cff += b.cff + df * df * k;
-  a.cgg += b.cgg + dg * dg * k;
-  a.cfg += b.cfg + df * dg * k;
-  a.mf += df * b.n / n;
-  a.mg += dg * b.n / n;
-  a.n = n;
+  a.n = warp_sum_d(a.n);
+  a.sm = warp_sum_d(a.sm);
+  a.sf = warp_sum_d(a.sf);
+  a.sg = warp_sum_d(a.sg);
+  a.mf = warp_sum_d(a.mf);
+  a.mg = warp_sum_d(a.mg);
+  if (!(a.n > 0)) return a;
+  a.mf /= a.n;
+  a.mg /= a.n;
+  for (int i = lane; i < nb; i += 32) {
+    const Moments* p = part + i;
+    const double n = __ldcg(&p->n), df = __ldcg(&p->mf) - a.mf, dg = __ldcg(&p->mg) - a.mg;
+    if (n > 0) {
+      a.cff += __ldcg(&p->cff) + n * df * df;
+      a.cgg += __ldcg(&p->cgg) + n * dg * dg;
+      a.cfg += __ldcg(&p->cfg) + n * df * dg;
+    }
+  }
+  a.cff = warp_sum_d(a.cff);
+  a.cgg = warp_sum_d(a.cgg);
+  a.cfg = warp_sum_d(a.cfg);
+  return a;
 }
 
 // ---- compensated FP32 sums ----
@@ -523,8 +597,14 @@ int gauss_1d(float radius, float* g, int cap);
 // Filter dispatch used by the plain operators and the engine set-up.
 int launch_filter(const asc_filter_desc& f, const float* in, float* out, int w, int h, cudaStream_t s);
 
-// One plain ray-cast launch with an already folded float matrix.
+// One plain ray-cast launch with an already folded float matrix; `merge`: its
+// DRR is added to what `out` holds and the sum held to 1 (asc_merge).
 int raycast_launch(const DevVolume& V, const uint8_t* clr, const float* m12, const float* vp, float step,
-                   float intensity, float cutoff, float* out, int w, int h, cudaStream_t s);
+                   float intensity, float cutoff, float* out, bool merge, int w, int h, cudaStream_t s);
+
+// The masks of trackFrame (Tracker.cpp:744-752) in one pass: mask = bg x (drr
+// != 0 ? 1 : 0) (bg null: ones), drr_out = drr x mask, rad_out = rad x mask.
+int mask_images(const float* drr, const float* rad, const float* bg, float* mask, float* drr_out, float* rad_out,
+                size_t n, cudaStream_t s);
 
 }  // namespace asc

@@ -642,7 +642,10 @@ __device__ __forceinline__ bool sample_above(const DevVolume& V, const RaySetup&
 // is never negative otherwise, see block_flagged), and the ray must be
 // marched again with EXACT true, which decides those samples with
 // sample_above.  cut is read only with EXACT.
-template <int STORE, bool EXACT>
+//
+// PAIRS: sample pairs whose loads are in flight together.  One where other
+// warps cover the loads; more where few warps are resident (they take registers).
+template <int STORE, bool EXACT, int PAIRS = 1>
 __device__ __forceinline__ float march_block(const DevVolume& V, const RaySetup& r, int kb, int js, int je,
                                               float lo, float hi, const Cutoff& cut)
 {
@@ -715,6 +718,25 @@ __device__ __forceinline__ float march_block(const DevVolume& V, const RaySetup&
     ib = min(__float_as_uint(tz.y) * pxy + __float_as_uint(ty.y) * px + __float_as_uint(tx.y) + i_base, imax);
   };
   int k = js;
+  if constexpr (PAIRS > 1)
+    for (; k + 2 * PAIRS - 1 <= je; k += 2 * PAIRS) {
+      float2 wx[PAIRS], wy[PAIRS], wz[PAIRS];
+      Taps<STORE> A[PAIRS], B[PAIRS];
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        unsigned ia, ib;
+        locate2(j + (float)(2 * p), wx[p], wy[p], wz[p], ia, ib);
+        A[p] = fetch_taps<STORE>(P, ia, px, pxy);
+        B[p] = fetch_taps<STORE>(P, ib, px, pxy);
+      }
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        const float2 v = trilinear2<STORE>(A[p], B[p], wx[p], wy[p], wz[p]);
+        take(v.x, kb + k + 2 * p);
+        take(v.y, kb + k + 2 * p + 1);
+      }
+      j += 2.0f * PAIRS;
+    }
   for (; k < je; k += 2) {
     float2 wx, wy, wz;
     unsigned ia, ib;

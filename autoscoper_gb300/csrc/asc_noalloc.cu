@@ -23,9 +23,8 @@ struct ReduceScratch {
   double* means;
   unsigned* ticket;
 };
-__global__ void __launch_bounds__(256) k_ncc(const float* __restrict__ f, const float* __restrict__ g,
-                                             const float* __restrict__ mask, unsigned n, int tree, ReduceScratch sc,
-                                             double* __restrict__ result);
+void launch_ncc(const float* f, const float* g, const float* mask, unsigned n, int tree, ReduceScratch sc,
+                double* result, cudaStream_t s);
 
 }  // namespace asc
 
@@ -118,9 +117,8 @@ ASC_API int asc_ncc_noalloc(const float* f, const float* g, const float* m, unsi
   ReduceScratch sc{(Moments*)b, (double*)(b + kPartBytes), (unsigned*)(b + kPartBytes + 2 * sizeof(double))};
   // the completion counter must start at zero; the partials are written before they are read
   ASC_CUDA(cudaMemsetAsync(sc.ticket, 0, sizeof(unsigned), S(stream)));
-  const unsigned blocks = (n + kChunk - 1) / kChunk;
   const int tree = coverage == ASC_SUM_TREE && tree_needed(n);
-  k_ncc<<<blocks, 256, 0, S(stream)>>>(f, g, m, n, tree, sc, res);
+  launch_ncc(f, g, m, n, tree, sc, res, S(stream));
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }

@@ -49,8 +49,10 @@ int gauss_1d(float radius, float* g, int cap)
 // ---------------------------------------------------------------- kernels
 
 // cuda_volume_render_kernel (RayCaster_kernels.cu:144-195) for one image: a
-// warp per beam of 8 x 4 pixels (ray_beam).  Rays with a sample in the
-// cutoff's band are marched again, exactly, by their warp.
+// warp, and a block, per beam of 8 x 4 pixels (ray_beam): most beams meet
+// nothing, and in a block of several the done ones would hold their warps' places until the
+// last is done.  Rays with a sample in the cutoff's band are marched again,
+// exactly, by their warp.  merge: the DRR is added to what `out` holds, held to 1.
 struct RayArgs {
   float m[12];
   float vp[4];
@@ -59,69 +61,87 @@ struct RayArgs {
   float sx[2], sy[2];  // vp[2] / w and vp[3] / h as double-floats
 };
 
-__global__ void __launch_bounds__(NRAY, 4) k_raycast(DevVolume V, const uint8_t* __restrict__ clr,
-                                                     const __grid_constant__ RayArgs a, float* __restrict__ out, int w,
-                                                     int h)
+// One image fills few warps, so two pairs of samples are in flight per lane
+// (96 registers): a 256 x 128 x 128 bone over 1024^2 58 us against 70 with one pair,
+// and 98-155 with a thread per ray walking by itself.
+constexpr int RAYCAST_PAIRS = 2;
+__global__ void __launch_bounds__(32, 20) k_raycast(DevVolume V, const uint8_t* __restrict__ clr,
+                                                    const __grid_constant__ RayArgs a, float* __restrict__ out,
+                                                    int merge, int y0, int w, int h)
 {
-  __shared__ RaySlots S;
-  __shared__ float s_v[NRAY / 32][EXACT_FLOATS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x, y;
-  beam_pixel(blockIdx.x * RTX, blockIdx.y * RTY, warp, 3, x, y);
+  __shared__ RaySlots<32> S;
+  __shared__ float s_v[EXACT_FLOATS];
+  const int lane = threadIdx.x;
+  const int x = blockIdx.x * 8 + (lane & 7), y = y0 + blockIdx.y * 4 + (lane >> 3);
   const bool valid = x < w && y < h;
   const RayScene s{a.m, a.vp, df{a.sx[0], a.sx[1]}, df{a.sy[0], a.sy[1]}, a.step, clr, w, h};
   const Beam b = beam_mask(V, s, min(x, w - 1), min(y, h - 1));
+  if (!b.mask && merge) return;  // adds nothing (a DRR lies in [0, 1])
   float d = 0.f;
   if (b.mask) {
     unsigned marched = 0, slots = 0;
-    d = ray_beam(V, s, a.cut, make_float4(a.cut.raw - a.cut.t0, a.cut.hi0 + a.cut.t0, a.cut.t1, 0.f), S, x, y, valid, b,
+    d = ray_beam<RAYCAST_PAIRS>(V, s, a.cut, make_float4(a.cut.raw - a.cut.t0, a.cut.hi0 + a.cut.t0, a.cut.t1, 0.f), S, x, y, valid, b,
                  marched, slots);
     for (unsigned m = __ballot_sync(FULL_WARP, valid && d != d); m; m &= m - 1) {
       const int q = __ffs(m) - 1;
       const int rx = __shfl_sync(FULL_WARP, x, q), ry = __shfl_sync(FULL_WARP, y, q);
-      const float e = march_exact(V, s, a.cut, rx, ry, s_v[warp]);
+      const float e = march_exact(V, s, a.cut, rx, ry, s_v);
       if (lane == q) d = e;
     }
   }
-  if (valid) out[(size_t)y * w + x] = fminf(fmaxf(d * a.scale, 0.f), 1.f);
+  if (!valid) return;
+  float* o = out + (size_t)y * w + x;
+  d = fminf(fmaxf(d * a.scale, 0.f), 1.f);
+  *o = merge ? fminf(*o + d, 1.0f) : d;
 }
 
 // image_render_kernel (RadRenderer_kernels.cu:85-116) and
 // background_render_kernel (BackgroundRenderer_kernels.cu:88-120).
 struct ImgArgs {
   float ip[4], vp[4];
+  double rw, rh, riw, rih;  // reciprocals of the image's and the image plane's sizes (image_axis)
   float threshold;
   int mode;  // 0 radiograph, 1 background mask
 };
 
-__global__ void __launch_bounds__(256) k_image_render(const void* __restrict__ img, int bps, int W, int H, ImgArgs a,
-                                                      float* __restrict__ out, int w, int h)
+// 64 x 32 pixels per block of 256.  What bounds it is FP64: the film-plane
+// mapping of a block's columns and rows (image_axis, 16 issue cycles an
+// operation and warp), shared by its pixels, so the blocks are large.
+// 1024^2: 24 us with 32 x 8 pixels per block and FP64 divisions, 10 here.
+constexpr int IW = 64, IH = 32;
+__global__ void __launch_bounds__(256) k_image_render(const void* __restrict__ img, int bps, int W, int H,
+                                                      const __grid_constant__ ImgArgs a, float* __restrict__ out, int w,
+                                                      int h)
 {
-  // the film-plane mapping of the block's 32 columns and 8 rows, in FP64
-  // (image_axis), shared by its pixels
-  __shared__ int s_k[40];
-  __shared__ float s_a[40];
-  const int t = threadIdx.y * 32 + threadIdx.x;
-  if (t < 40) {
-    const bool row = t >= 32;
-    const int j = row ? blockIdx.y * 8 + (t - 32) : blockIdx.x * 32 + t;
+  __shared__ int s_k[IW + IH];
+  __shared__ float s_a[IW + IH];
+  const int t = threadIdx.x, x0 = blockIdx.x * IW, y0 = blockIdx.y * IH;
+  if (t < IW + IH) {
+    const bool row = t >= IW;
+    const int j = row ? y0 + (t - IW) : x0 + t;
     int k = 0;
     float wgt = 0.f;
-    const bool ok = row ? j < h && image_axis(a.vp[1], a.vp[3], j, h, a.ip[1], a.ip[3], H, true, k, wgt)
-                        : j < w && image_axis(a.vp[0], a.vp[2], j, w, a.ip[0], a.ip[2], W, false, k, wgt);
+    const bool ok =
+        row ? j < h && image_axis(a.vp[1], a.vp[3], j, h, a.rh, a.ip[1], a.ip[3], a.rih, H, true, k, wgt)
+            : j < w && image_axis(a.vp[0], a.vp[2], j, w, a.rw, a.ip[0], a.ip[2], a.riw, W, false, k, wgt);
     s_k[t] = ok ? k : INT_MIN;
     s_a[t] = wgt;
   }
   __syncthreads();
-  int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-  if (x >= w || y >= h) return;
-  const int kx = s_k[threadIdx.x], ky = s_k[32 + threadIdx.y];
-  float r = 0.f;
-  if (kx != INT_MIN && ky != INT_MIN) {
-    float v = bilinear_at(img, bps, W, H, kx, s_a[threadIdx.x], ky, s_a[32 + threadIdx.y]);
-    r = a.mode == 0 ? 1.0f - v : (a.threshold <= v ? 1.0f : 0.0f);
+  const int lx = t % IW, x = x0 + lx, kx = s_k[lx];
+  const float ax = s_a[lx];
+  if (x >= w) return;
+#pragma unroll
+  for (int ly = t / IW; ly < IH; ly += 256 / IW) {
+    const int y = y0 + ly, ky = s_k[IW + ly];
+    if (y >= h) return;
+    float r = 0.f;
+    if (kx != INT_MIN && ky != INT_MIN) {
+      const float v = bilinear_at(img, bps, W, H, kx, ax, ky, s_a[IW + ly]);
+      r = a.mode == 0 ? 1.0f - v : (a.threshold <= v ? 1.0f : 0.0f);
+    }
+    out[(size_t)y * w + x] = r;
   }
-  out[(size_t)y * w + x] = r;
 }
 
 // Elementwise operators (DRRBackground / Mult / Merger / Compositor kernels).
@@ -132,7 +152,7 @@ __global__ void k_elementwise(int op, const float* __restrict__ a, const float* 
     switch (op) {
       case 0: d[i] = a[i] != 0.0f ? 1.0f : 0.0f; break;
       case 1: d[i] = a[i] * b[i]; break;
-      case 2: d[i] = (float)fmin((double)(a[i] + b[i]), 1.0); break;
+      case 2: d[i] = fminf(a[i] + b[i], 1.0f); break;
       case 3: {
         float multi = c[i] < 0.5f ? 0.0f : 1.0f;
         float s1 = a[i], s2 = b[i];
@@ -144,6 +164,27 @@ __global__ void k_elementwise(int op, const float* __restrict__ a, const float* 
       default: d[i] = val; break;
     }
   }
+}
+
+// trackFrame's masks (mask_images), where four elementwise launches moved 44 bytes a pixel instead of 24.
+__global__ void __launch_bounds__(256) k_mask(const float* drr, const float* rad, const float* bg, float* mask,
+                                              float* drr_out, float* rad_out, size_t n)
+{
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const float d = drr[i], r = rad[i], seen = d != 0.0f ? 1.0f : 0.0f, m = bg ? bg[i] * seen : seen;
+    mask[i] = m;
+    rad_out[i] = r * m;
+    drr_out[i] = d * m;
+  }
+}
+
+int mask_images(const float* drr, const float* rad, const float* bg, float* mask, float* drr_out, float* rad_out,
+                size_t n, cudaStream_t s)
+{
+  if (n == 0) return ASC_OK;
+  k_mask<<<(int)std::min<size_t>((n + 255) / 256, 152 * 16), 256, 0, s>>>(drr, rad, bg, mask, drr_out, rad_out, n);
+  ASC_LAUNCH_CHECK();
+  return ASC_OK;
 }
 
 // ---- 2-D stencil filters, 32x32 output tiles staged in shared memory ----
@@ -228,6 +269,121 @@ __global__ void __launch_bounds__(256) k_stencil(const float* __restrict__ in, f
   }
 }
 
+// The filters of usual size with the taps and the staged tile's edges known to
+// the compiler: no index division by the edge, the taps from the constant
+// bank, and a warp's lanes on 32 columns of four rows, whose windows overlap
+// (a 7-tap vertical pass reads 10 words for 4 outputs).  The same operations per pixel, in the same order,
+// as k_stencil.  Sobel stages its neighbours outside the image as the edge's.
+// What bounds them is launch and load latency (4 MB in and out of L2 at 1021 x
+// 983, and for Contrast its two powf): Contrast 18.0, Sharpen 12.1, Gaussian
+// 12.4, Sobel 10.0 us with k_stencil; 13.2, 7.4, 7.6 and 6.0 here.
+constexpr int FR = 4;  // rows per warp
+template <int KIND, int K>
+__global__ void __launch_bounds__(256) k_filter(const float* __restrict__ in, float* __restrict__ out, int w, int h,
+                                                const __grid_constant__ StencilArgs a)
+{
+  constexpr int R = K / 2, E = FT + 2 * R;
+  constexpr bool BLUR = KIND == 3 || KIND == 4;
+  __shared__ float tile[E][E + 1];
+  __shared__ float hp[BLUR ? E : 1][FT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * FT - R, y0 = blockIdx.y * FT - R;
+#pragma unroll
+  for (int j = 0; j < (E + 7) / 8; ++j) {
+    const int ty = warp + 8 * j;
+    if (ty < E)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int tx = lane + 32 * c;
+        if (tx < E) {
+          int x = x0 + tx, y = y0 + ty;
+          float v = 0.f;
+          if (KIND == 1) {
+            x = min(max(x, 0), w - 1);
+            y = min(max(y, 0), h - 1);
+          }
+          if (KIND == 1 || (x >= 0 && x < w && y >= 0 && y < h)) v = __ldg(in + (size_t)y * w + x);
+          tile[ty][tx] = v;
+        }
+      }
+  }
+  __syncthreads();
+  if (BLUR) {
+#pragma unroll
+    for (int j = 0; j < (E + 7) / 8; ++j) {
+      const int ty = warp + 8 * j;
+      if (ty < E) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) s = fmaf(a.g[k], tile[ty][lane + k], s);
+        hp[ty][lane] = s;
+      }
+    }
+    __syncthreads();
+  }
+  const int gx = blockIdx.x * FT + lane, gy0 = blockIdx.y * FT + warp * FR;
+  if (gx >= w) return;
+  float col[BLUR ? K + FR - 1 : 1];
+  if (BLUR)
+#pragma unroll
+    for (int t = 0; t < K + FR - 1; ++t) col[t] = hp[warp * FR + t][lane];
+#pragma unroll
+  for (int t = 0; t < FR; ++t) {
+    const int gy = gy0 + t, ty = warp * FR + t;
+    if (gy >= h) return;
+    const float f = tile[ty + R][lane + R];
+    float r;
+    if (BLUR) {
+      float blur = 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k) blur = fmaf(a.g[k], col[t + k], blur);
+      if (KIND == 3)
+        r = fminf(fmaxf(blur, 0.f), 1.f);
+      else
+        r = fabsf(f - blur) > a.p2 ? fminf(fmaxf(f + a.p1 * (f - blur), 0.f), 1.f) : f;
+    } else if (KIND == 1) {
+      const float p00 = tile[ty][lane], p01 = tile[ty][lane + 1], p02 = tile[ty][lane + 2];
+      const float p10 = tile[ty + 1][lane], p12 = tile[ty + 1][lane + 2];
+      const float p20 = tile[ty + 2][lane], p21 = tile[ty + 2][lane + 1], p22 = tile[ty + 2][lane + 2];
+      const float horz = p02 + 2 * p12 + p22 - p00 - 2 * p10 - p20;
+      const float vert = p00 + 2 * p01 + p02 - p20 - 2 * p21 - p22;
+      const float grad = sqrtf(horz * horz + vert * vert);
+      const float s = a.p1 < 0.5f ? a.p0 * grad + 2.0f * a.p1 * f : 2.0f * (1.0f - a.p1) * a.p0 * grad + f;
+      r = fminf(fmaxf(s, 0.f), 1.f);
+    } else {
+      float s = 0.f;
+#pragma unroll
+      for (int yy = 0; yy < K; ++yy)
+#pragma unroll
+        for (int xx = 0; xx < K; ++xx) s += tile[ty + yy][lane + xx];  // 0 outside the image
+      float axy;
+      if (K == 3 && gx > 0 && gx < w - 1 && gy > 0 && gy < h - 1) {
+        axy = ninth(s);
+      } else {
+        const int ny = min(gy + (K + 1) / 2, h) - max(gy - R, 0), nx = min(gx + (K + 1) / 2, w) - max(gx - R, 0);
+        axy = s / (float)(ny * nx);
+      }
+      r = axy > 0.01f ? powf(axy, a.p0 - a.p1) * powf(f, a.p1) : 0.0f;
+    }
+    out[(size_t)gy * w + gx] = r;
+  }
+}
+
+using FilterKernel = void (*)(const float*, float*, int, int, StencilArgs);
+template <int KIND>
+static FilterKernel blur_kernel(int K)
+{
+  switch (K) {
+    case 3: return k_filter<KIND, 3>;
+    case 5: return k_filter<KIND, 5>;
+    case 7: return k_filter<KIND, 7>;
+    case 9: return k_filter<KIND, 9>;
+    case 11: return k_filter<KIND, 11>;
+    case 13: return k_filter<KIND, 13>;
+  }
+  return nullptr;  // k_stencil
+}
+
 // ---- cost reductions ----
 constexpr int RB = 256;          // threads per reduction block
 constexpr int RE = 16;           // elements per thread
@@ -274,83 +430,114 @@ struct ReduceScratch {
   unsigned* ticket;     // last-block election
 };
 
-// Merges `nb` partials in FP64 with one block; returns the result in m (thread 0).
-__device__ void merge_partials(const Moments* part, int nb, Moments& m)
-{
-  __shared__ Moments sh[RB];
-  Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) moments_merge(a, part[i]);
-  sh[threadIdx.x] = a;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) moments_merge(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
-  m = sh[0];
-}
-
 // NCC (Ncc_kernels.cu:116-213) in one launch: each block computes the
 // moments of its 4096 elements in two passes over registers, the last block
-// to finish merges all partials in FP64 and writes the correlation.
-__global__ void __launch_bounds__(RB) k_ncc(const float* __restrict__ f, const float* __restrict__ g,
+// to finish merges all partials in FP64 and writes the correlation.  What
+// bounds it is latency: the load, two compensated block sums, then the FP64
+// tail of the last block; so a block has 1024 threads of 4 elements, each
+// block sum is finished by a warp per value, and one warp merges.  120 000
+// pixels: 31 us with 256 threads of 16 elements and a pairwise merge, 16 here.
+constexpr int NT = 1024, NE = RCHUNK / NT;
+template <int N>
+__device__ __forceinline__ void wide_sum_dfs(DFs (&v)[N], float2 (*red)[NT / 32], double* out)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      DFs b = {__shfl_xor_sync(FULL_WARP, v[k].h, o), __shfl_xor_sync(FULL_WARP, v[k].l, o)};
+      dfs_merge(v[k], b);
+    }
+    if (lane == 0) red[k][warp] = make_float2(v[k].h, v[k].l);
+  }
+  __syncthreads();
+  if (warp < N) {
+    const float2 p = red[warp][lane];
+    const double t = warp_sum_d((double)p.x + (double)p.y);
+    if (lane == 0) out[warp] = t;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const float* __restrict__ g,
                                             const float* __restrict__ mask, unsigned n, int tree, ReduceScratch sc,
                                             double* __restrict__ result)
 {
-  __shared__ float red[(RB / 32) * 6 * 2];
+  __shared__ float2 red[6][NT / 32];
   __shared__ double ds[6], dc[3];
-  __shared__ bool last;
-  float fv[RE], gv[RE], mv[RE];
-  unsigned flags = 0;  // bit k: covered; bit 16+k: covered and mask > 0.5
+  __shared__ float s_mean[2];
+  __shared__ unsigned s_keep[8];
+  float fv[NE], gv[NE], mv[NE];
+  unsigned flags = 0;  // bit k: covered and mask > 0.5
   const size_t base = (size_t)blockIdx.x * RCHUNK + threadIdx.x;
-  DFs s[6] = {};  // sm, sf, sg (covered), n, sf, sg (masked)
 #pragma unroll
-  for (int k = 0; k < RE; ++k) {
-    size_t i = base + (size_t)k * RB;
+  for (int k = 0; k < NE; ++k) {
+    const size_t i = base + (size_t)k * NT;
     fv[k] = gv[k] = mv[k] = 0.f;
-    if (i < n && (!tree || tree_keep((unsigned)i, n))) {
+    if (i < n) {
       fv[k] = __ldg(f + i);
       gv[k] = __ldg(g + i);
       mv[k] = __ldg(mask + i);
-      flags |= 1u << k;
+    }
+  }
+  int shift = 0;
+  if (tree) {
+    if (threadIdx.x < 256) shift = tree_mask(n, s_keep);
+    for (unsigned m = n; threadIdx.x >= 256 && m > 256u; m = (m + 255u) >> 8) shift += 8;
+    __syncthreads();
+  }
+  DFs s[6] = {};  // sm, sf, sg (covered), n, sf, sg (masked)
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const size_t i = base + (size_t)k * NT;
+    if (i < n && (!tree || tree_kept(s_keep, (unsigned)i, shift))) {
       dfs_add(s[0], mv[k]);
       dfs_add(s[1], fv[k]);
       dfs_add(s[2], gv[k]);
       if (mv[k] > 0.5f) {
-        flags |= 1u << (16 + k);
+        flags |= 1u << k;
         dfs_add(s[3], 1.f);
         dfs_add(s[4], fv[k]);
         dfs_add(s[5], gv[k]);
       }
     }
   }
-  block_sum_dfs<6>(s, red, ds);
-  const double cnt = ds[3];
-  const float mf = cnt > 0 ? (float)(ds[4] / cnt) : 0.f, mg = cnt > 0 ? (float)(ds[5] / cnt) : 0.f;
+  wide_sum_dfs<6>(s, red, ds);
+  if (threadIdx.x < 2) s_mean[threadIdx.x] = ds[3] > 0 ? (float)(ds[4 + threadIdx.x] / ds[3]) : 0.f;
+  __syncthreads();
+  const float mf = s_mean[0], mg = s_mean[1];
   DFs c[3] = {};
 #pragma unroll
-  for (int k = 0; k < RE; ++k)
-    if (flags & (1u << (16 + k))) {
+  for (int k = 0; k < NE; ++k)
+    if (flags & (1u << k)) {
       float a = fv[k] - mf, b = gv[k] - mg;
       dfs_add_prod(c[0], a, a);
       dfs_add_prod(c[1], b, b);
       dfs_add_prod(c[2], a, b);
     }
-  block_sum_dfs<3>(c, red, dc);
+  wide_sum_dfs<3>(c, red, dc);
+  if (threadIdx.x >= 32) return;
+  bool last = false;
   if (threadIdx.x == 0) {
-    Moments p = tile_moments(ds, dc, mf, mg);
-    sc.part[blockIdx.x] = p;
+    sc.part[blockIdx.x] = tile_moments(ds, dc, mf, mg);
     __threadfence();
     last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
   }
-  __syncthreads();
-  if (!last) return;
+  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
   __threadfence();
-  Moments m;
-  merge_partials(sc.part, gridDim.x, m);
+  const Moments m = merge_moments(sc.part, gridDim.x);
   if (threadIdx.x == 0) {
     *result = moments_ncc(m);
     *sc.ticket = 0;
   }
+}
+
+// The launch for n elements, the same for asc_ncc and asc_ncc_noalloc.
+void launch_ncc(const float* f, const float* g, const float* mask, unsigned n, int tree, ReduceScratch sc,
+                double* result, cudaStream_t s)
+{
+  k_ncc<<<(unsigned)(((size_t)n + RCHUNK - 1) / RCHUNK), NT, 0, s>>>(f, g, mask, n, tree, sc, result);
 }
 
 // SAD ("hdist", HDist_kernels.cu:111-203): pass 1 computes the masked means
@@ -360,29 +547,35 @@ __global__ void __launch_bounds__(RB) k_hdist_means(const float* __restrict__ f,
                                                     ReduceScratch sc)
 {
   __shared__ float red[(RB / 32) * 3];
-  __shared__ bool last;
+  __shared__ unsigned s_keep[RB / 32];
   float s[3] = {0, 0, 0};
   const size_t base = (size_t)blockIdx.x * RCHUNK + threadIdx.x;
+  int shift = 0;
+  if (tree) {
+    shift = tree_mask(n, s_keep);
+    __syncthreads();
+  }
+#pragma unroll
   for (int k = 0; k < RE; ++k) {
     size_t i = base + (size_t)k * RB;
-    if (i < n && (!tree || tree_keep((unsigned)i, n))) {
+    if (i < n && (!tree || tree_kept(s_keep, (unsigned)i, shift))) {
       s[0] += __ldg(mask + i);
       s[1] += __ldg(f + i);
       s[2] += __ldg(g + i);
     }
   }
   block_sum<3>(s, red);
+  if (threadIdx.x >= 32) return;
+  bool last = false;
   if (threadIdx.x == 0) {
     Moments p = {s[0], s[1], s[2], 0, 0, 0, 0, 0, 0};
     sc.part[blockIdx.x] = p;
     __threadfence();
     last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
   }
-  __syncthreads();
-  if (!last) return;
+  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
   __threadfence();
-  Moments m;
-  merge_partials(sc.part, gridDim.x, m);
+  const Moments m = merge_moments(sc.part, gridDim.x);
   if (threadIdx.x == 0) {
     sc.means[0] = m.sf / m.sm;
     sc.means[1] = m.sg / m.sm;
@@ -395,27 +588,33 @@ __global__ void __launch_bounds__(RB) k_hdist_sad(const float* __restrict__ f, c
                                                   ReduceScratch sc, double* __restrict__ result)
 {
   __shared__ float red[RB / 32];
-  __shared__ bool last;
+  __shared__ unsigned s_keep[RB / 32];
   const float mF = (float)sc.means[0], mG = (float)sc.means[1];
   float s[1] = {0};
   const size_t base = (size_t)blockIdx.x * RCHUNK + threadIdx.x;
+  int shift = 0;
+  if (tree) {
+    shift = tree_mask(n, s_keep);
+    __syncthreads();
+  }
+#pragma unroll
   for (int k = 0; k < RE; ++k) {
     size_t i = base + (size_t)k * RB;
-    if (i < n && (!tree || tree_keep((unsigned)i, n)) && __ldg(mask + i) > 0.5f)
+    if (i < n && (!tree || tree_kept(s_keep, (unsigned)i, shift)) && __ldg(mask + i) > 0.5f)
       s[0] += fabsf((__ldg(f + i) - mF) - (__ldg(g + i) - mG));
   }
   block_sum<1>(s, red);
+  if (threadIdx.x >= 32) return;
+  bool last = false;
   if (threadIdx.x == 0) {
     Moments p = {s[0], 0, 0, 0, 0, 0, 0, 0, 0};
     sc.part[blockIdx.x] = p;
     __threadfence();
     last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
   }
-  __syncthreads();
-  if (!last) return;
+  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
   __threadfence();
-  Moments m;
-  merge_partials(sc.part, gridDim.x, m);
+  const Moments m = merge_moments(sc.part, gridDim.x);
   if (threadIdx.x == 0) {
     *result = m.sm;
     *sc.ticket = 0;
@@ -541,11 +740,22 @@ int launch_filter(const asc_filter_desc& f, const float* in, float* out, int w, 
   } else {
     return ASC_ERR_ARG;
   }
+  const dim3 grid((w + FT - 1) / FT, (h + FT - 1) / FT);
+  const FilterKernel fast = f.kind == 1   ? k_filter<1, 3>
+                            : f.kind == 3 ? blur_kernel<3>(a.K)
+                            : f.kind == 4 ? blur_kernel<4>(a.K)
+                            : a.K == 3    ? k_filter<0, 3>
+                            : a.K == 5    ? k_filter<0, 5>
+                                          : nullptr;
+  if (fast) {
+    fast<<<grid, 256, 0, s>>>(in, out, w, h, a);
+    ASC_LAUNCH_CHECK();
+    return ASC_OK;
+  }
   int E = FT + 2 * R;
   size_t smem = (size_t)(E * E + E * FT) * sizeof(float);
   static std::once_flag once;
   std::call_once(once, [] { cudaFuncSetAttribute(k_stencil, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
-  dim3 grid((w + FT - 1) / FT, (h + FT - 1) / FT);
   k_stencil<<<grid, 256, smem, s>>>(in, out, w, h, a);
   ASC_LAUNCH_CHECK();
   return ASC_OK;
@@ -904,7 +1114,7 @@ ASC_API int asc_volume_destroy(asc_volume vol)
 
 namespace asc {
 int raycast_launch(const DevVolume& V, const uint8_t* clr, const float* m12, const float* vp, float step,
-                   float intensity, float cutoff, float* out, int w, int h, cudaStream_t s)
+                   float intensity, float cutoff, float* out, bool merge, int w, int h, cudaStream_t s)
 {
   RayArgs a;
   memcpy(a.m, m12, sizeof a.m);
@@ -915,8 +1125,11 @@ int raycast_launch(const DevVolume& V, const uint8_t* clr, const float* m12, con
   a.cut = make_cutoff(cutoff, V.norm, V.gmax);
   df_split((double)vp[2] / (double)w, a.sx[0], a.sx[1]);
   df_split((double)vp[3] / (double)h, a.sy[0], a.sy[1]);
-  dim3 grid((w + RTX - 1) / RTX, (h + RTY - 1) / RTY);
-  k_raycast<<<grid, NRAY, 0, s>>>(V, clr, a, out, w, h);
+  // the grid's rows reach 65535: taller images take several launches
+  for (int y0 = 0; y0 < h; y0 += 4 * 65535) {
+    const dim3 grid((w + 7) / 8, std::min((h - y0 + 3) / 4, 65535));
+    k_raycast<<<grid, 32, 0, s>>>(V, clr, a, out, merge, y0, w, h);
+  }
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }
@@ -949,7 +1162,7 @@ ASC_API int asc_raycast(asc_volume vol, const double imv[16], const float vp[4],
     }
     clr = v->clr;
   }
-  return raycast_launch(v->dev, clr, m, vp, step, intensity, cutoff, out, w, h, S(stream));
+  return raycast_launch(v->dev, clr, m, vp, step, intensity, cutoff, out, false, w, h, S(stream));
 }
 
 // ---- images ----
@@ -1041,8 +1254,12 @@ static int image_render(asc_image im, const float ip[4], const float vp[4], int 
   memcpy(a.vp, vp, sizeof a.vp);
   a.threshold = thr;
   a.mode = mode;
-  dim3 b(32, 8), g((w + 31) / 32, (h + 7) / 8);
-  k_image_render<<<g, b, 0, S(stream)>>>(im->data, im->bps, im->w, im->h, a, out, w, h);
+  a.rw = reciprocal((double)w);
+  a.rh = reciprocal((double)h);
+  a.riw = reciprocal((double)ip[2]);
+  a.rih = reciprocal((double)ip[3]);
+  const dim3 g((w + IW - 1) / IW, (h + IH - 1) / IH);
+  k_image_render<<<g, 256, 0, S(stream)>>>(im->data, im->bps, im->w, im->h, a, out, w, h);
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }
@@ -1136,7 +1353,7 @@ int asc::ncc_init_locked(unsigned max_n)
   g_ticket = nullptr;
   g_max_n = 0;
   if (max_n == 0) return ASC_OK;
-  size_t nb = (max_n + RCHUNK - 1) / RCHUNK;
+  const size_t nb = ((size_t)max_n + RCHUNK - 1) / RCHUNK;
   ASC_CUDA(cudaMalloc(&g_part, nb * sizeof(Moments)));
   ASC_CUDA(cudaMalloc(&g_means, 2 * sizeof(double)));
   ASC_CUDA(cudaMalloc(&g_ticket, sizeof(unsigned)));
@@ -1153,7 +1370,7 @@ ASC_API int asc_ncc(const float* f, const float* g, const float* m, unsigned n, 
   int rc = ensure_scratch(n, &sc);
   if (rc) return rc;
   int tree = coverage == ASC_SUM_TREE && tree_needed(n);
-  k_ncc<<<(n + RCHUNK - 1) / RCHUNK, RB, 0, S(st)>>>(f, g, m, n, tree, sc, res);
+  launch_ncc(f, g, m, n, tree, sc, res, S(st));
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }

@@ -93,8 +93,9 @@ __device__ __forceinline__ Beam beam_mask(const DevVolume& V, const RayScene& s,
 
 // A ray's set-up, kept in the thread's own slots of shared memory: the march
 // of a segment reads it once, and in registers it would spill.
+template <int THREADS>
 struct RaySlots {
-  float4 q[3][NRAY];  // X, Y, Z, dX, dY, dZ as double-floats
+  float4 q[3][THREADS];  // X, Y, Z, dX, dY, dZ as double-floats
 };
 
 // A ray's place in its beam's runs: the intervals left, the samples
@@ -113,7 +114,8 @@ struct RunState {
 // box per 8-voxel cell did (39.1 against 38.2 a ray on the benchmark's bones,
 // none 47.2, two 40.8).
 constexpr int TRIMS = 4;
-__device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* __restrict__ clr, const RaySlots& S,
+template <class Slots>
+__device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* __restrict__ clr, const Slots& S,
                                              int K, float tf, const Beam& b, RunState& s, int& kb, int& js, int& je)
 {
   for (;;) {
@@ -167,8 +169,8 @@ __device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* 
 // The segments of this lane's ray (K samples; 0: none), marched side by side
 // with the warp's other lanes.  Returns their sum in raw units: NaN when a
 // sample fell in the cutoff's band.
-template <int STORE>
-__device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* __restrict__ clr, const RaySlots& S,
+template <int STORE, int PAIRS, class Slots>
+__device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* __restrict__ clr, const Slots& S,
                                             int K, float tf, const Beam& b, float4 band, const Cutoff& cut,
                                             unsigned& marched, unsigned& slots)
 {
@@ -188,7 +190,7 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
       r.dZ = df{q2.z, q2.w};
       // this ray's band: raw - t0, hi0 + t0 and t1 (cutoff_bounds)
       const float D = fabsf(q1.z) + fabsf(q2.x) + fabsf(q2.z);
-      const float p = march_block<STORE, false>(V, r, kb, js, je, fmaf(-band.z, D, band.x), fmaf(band.z, D, band.y), cut);
+      const float p = march_block<STORE, false, PAIRS>(V, r, kb, js, je, fmaf(-band.z, D, band.x), fmaf(band.z, D, band.y), cut);
       if (block_flagged(p))
         total.h = __int_as_float(0x7fffffff);  // NaN stays NaN through add_block
       else
@@ -205,8 +207,9 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
 
 // The DRR sum of the ray at pixel (x, y) (valid: inside the image) of this
 // warp's beam.  band: the cutoff's raw - t0, hi0 + t0 and t1.
+template <int PAIRS, class Slots>
 __device__ __forceinline__ float ray_beam(const DevVolume& V, const RayScene& s, const Cutoff& cut, float4 band,
-                                          RaySlots& S, int x, int y, bool valid, const Beam& b, unsigned& marched,
+                                          Slots& S, int x, int y, bool valid, const Beam& b, unsigned& marched,
                                           unsigned& slots)
 {
   int K = 0;
@@ -221,10 +224,10 @@ __device__ __forceinline__ float ray_beam(const DevVolume& V, const RayScene& s,
       tf = r.tf;
     }
   }
-  if (V.storage == ASC_STORE_F32) return march_beam<ASC_STORE_F32>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
-  if (V.storage == ASC_STORE_BF16) return march_beam<ASC_STORE_BF16>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
-  if (V.storage == ASC_STORE_F16) return march_beam<ASC_STORE_F16>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
-  return march_beam<ASC_STORE_U16>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
+  if (V.storage == ASC_STORE_F32) return march_beam<ASC_STORE_F32, PAIRS>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
+  if (V.storage == ASC_STORE_BF16) return march_beam<ASC_STORE_BF16, PAIRS>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
+  if (V.storage == ASC_STORE_F16) return march_beam<ASC_STORE_F16, PAIRS>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
+  return march_beam<ASC_STORE_U16, PAIRS>(V, s.clr, S, K, tf, b, band, cut, marched, slots);
 }
 
 // The DRR sum of one ray (raw units) by one warp, every cutoff decision the

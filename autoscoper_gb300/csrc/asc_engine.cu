@@ -141,10 +141,16 @@ struct Bufs {
   Counters* C;
 };
 
-__device__ void finish_item(const SceneDev* sc, const Bufs& b, int item, double* cost)
+// The last view of an item is scored: its cost, and its views' costs.
+__device__ void finish_item(const SceneDev* sc, const Bufs& b, int item, double* cost, double* view_cost_out)
 {
+  const int ns = sc->slots;
   double tot = 0;
-  for (int j = 0; j < sc->slots; ++j) tot += b.vcost[item * sc->slots + j];
+  for (int j = 0; j < ns; ++j) {
+    const double v = b.vcost[item * ns + j];
+    tot += v;
+    if (view_cost_out) view_cost_out[item * ns + j] = v;
+  }
   cost[item] = tot < 0 ? 9999.0 : tot;  // Tracker.cpp:823-825
 }
 
@@ -474,7 +480,8 @@ __device__ __forceinline__ void warp_fill(int* __restrict__ p, int from, int to,
 __global__ void __launch_bounds__(SETUP_THREADS) k_setup(const SceneDev* __restrict__ sc, int n_items,
                                                          const int* __restrict__ bone_in,
                                                          const double* __restrict__ manip, Bufs b,
-                                                         double* __restrict__ cost)
+                                                         double* __restrict__ cost, double* __restrict__ view_cost_out,
+                                                         int* __restrict__ error_out)
 {
   __shared__ SetupWarp s_w;
   __shared__ long long s_scan[3][SETUP_THREADS / 32];
@@ -545,6 +552,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_setup(const SceneDev* __restr
     b.C->rnext = 0;
     b.C->fnext = 0;
     b.C->error = s_err;
+    if (error_out) *error_out = s_err;
     b.C->nfix = 0;
     b.C->nfixb = 0;
     b.C->samples = 0;
@@ -558,7 +566,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_setup(const SceneDev* __restr
     unsigned pre = 0;
     for (int v = 0; v < nv; ++v) pre += __ldcg(&b.iv[item * nv + v].ok) ? 0u : 1u;
     b.itt[item] = pre;
-    if (pre == (unsigned)nv) finish_item(sc, b, item, cost);
+    if (pre == (unsigned)nv) finish_item(sc, b, item, cost, view_cost_out);
   }
 }
 
@@ -1233,9 +1241,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     const int item = k / ns;
     if (atomicAdd(&b.itt[item], 1u) == (unsigned)ns - 1) {
       __threadfence();
-      finish_item(sc, b, item, cost);
-      if (view_cost_out)
-        for (int j = 0; j < ns; ++j) view_cost_out[item * ns + j] = b.vcost[item * ns + j];
+      finish_item(sc, b, item, cost, view_cost_out);
     }
   }
 }
@@ -1297,19 +1303,12 @@ __global__ void __launch_bounds__(256) k_sad(const SceneDev* __restrict__ sc, Bu
         const int item = k / nv;
         if (atomicAdd(&b.itt[item], 1u) == (unsigned)nv - 1) {
           __threadfence();
-          finish_item(sc, b, item, cost);
-          if (view_cost_out)
-            for (int j = 0; j < nv; ++j) view_cost_out[item * nv + j] = b.vcost[item * nv + j];
+          finish_item(sc, b, item, cost, view_cost_out);
         }
       }
     }
     __syncthreads();
   }
-}
-
-// Copies view costs of items finished entirely in k_setup.
-__global__ void k_copy_vcost(const double* vc, double* out, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = vc[i];
 }
 
 // ---------------------------------------------------------------- PSO
@@ -1427,6 +1426,13 @@ __global__ void k_pso_best(Swarm s, int nb, int np, const double* cost)
 
 // ---------------------------------------------------------------- host side
 
+// asc_engine_eval_host's staging, pinned host memory sized for max_items.
+struct HostIO {
+  void* base = nullptr;
+  double *manip = nullptr, *cost = nullptr, *vcost = nullptr;
+  int *bone = nullptr, *error = nullptr;
+};
+
 struct asc_engine_s {
   SceneDev host;
   SceneDev* dev = nullptr;
@@ -1456,7 +1462,7 @@ struct asc_engine_s {
   int* d_bone = nullptr;
   double* d_manip = nullptr;
   double* d_cost = nullptr;
-  double* d_vcost = nullptr;
+  HostIO io;
   // plain per-pose path: the reference's Tracker buffers (Tracker.cpp:292-298)
   std::vector<asc_view_desc> vdesc;
   std::vector<asc_bone_desc> bdesc;
@@ -1470,6 +1476,7 @@ struct asc_engine_s {
   ~asc_engine_s()
   {
     for (void* p : allocs) cudaFree(p);
+    if (io.base) cudaFreeHost(io.base);
     for (auto& row : clr_own)
       for (uint8_t* p : row)
         if (p) cudaFree(p);
@@ -1673,7 +1680,16 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
   if (!err) err = e->alloc(e->d_bone, (size_t)max_items);
   if (!err) err = e->alloc(e->d_manip, (size_t)max_items * 6);
   if (!err) err = e->alloc(e->d_cost, (size_t)max_items);
-  if (!err) err = e->alloc(e->d_vcost, n_iv);
+  if (!err) err = cudaMallocHost(&e->io.base, (max_items * (size_t)(7 + S.slots)) * sizeof(double) +
+                                                   (max_items + (size_t)1) * sizeof(int));
+  if (!err) {
+    HostIO& io = e->io;
+    io.manip = (double*)io.base;
+    io.cost = io.manip + 6 * (size_t)max_items;
+    io.vcost = io.cost + max_items;
+    io.bone = (int*)(io.vcost + n_iv);
+    io.error = io.bone + max_items;
+  }
   const size_t npix = (size_t)rw * rh;
   if (!err) err = e->alloc(e->p_drr, npix);
   if (!err) err = e->alloc(e->p_rad, npix);
@@ -1935,11 +1951,11 @@ ASC_API int asc_engine_get_launch(asc_engine e, asc_launch_config* cfg, int* vie
 }
 
 static int engine_launch(asc_engine e, int n, const int* bone, const double* manip, double* cost, double* vcost,
-                         cudaStream_t s, bool capturing = false)
+                         cudaStream_t s, bool capturing = false, int* error = nullptr)
 {
   const bool prof = e->prof && !capturing;
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[0], s));
-  k_setup<<<n, SETUP_THREADS, 0, s>>>(e->dev, n, bone, manip, e->b, cost);
+  k_setup<<<n, SETUP_THREADS, 0, s>>>(e->dev, n, bone, manip, e->b, cost, vcost, error);
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[1], s));
   k_ray<<<e->sms * e->launch.ray_blocks_per_sm, NRAY, 0, s>>>(e->dev, e->b, g_empty_skip, e->launch.ray_shape);
   k_ray_fix<<<e->sms * 4, FIX_THREADS, 0, s>>>(e->dev, e->b, e->launch.ray_shape);
@@ -1947,7 +1963,6 @@ static int engine_launch(asc_engine e, int n, const int* bone, const double* man
   k_view<<<e->sms * e->view_grid(), VNT, e->smem, s>>>(e->dev, e->b, cost, vcost);
   if (e->host.cf_model) k_sad<<<e->sms * 8, 256, 0, s>>>(e->dev, e->b, cost, vcost);
   if (prof) ASC_CUDA(cudaEventRecord(e->ev[3], s));
-  if (vcost) k_copy_vcost<<<8, 256, 0, s>>>(e->b.vcost, vcost, n * e->host.slots);
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }
@@ -2020,18 +2035,20 @@ ASC_API int asc_engine_eval_host(asc_engine e, int n, const int* bone, const dou
                                  double* vcost, void* stream)
 {
   if (!e || !bone || !manip || !cost || n < 1 || n > e->max_items) return ASC_ERR_ARG;
+  // the candidates and the results pass through pinned host memory that the
+  // kernels read and write themselves: they are a few KB, and two copies in,
+  // three out of pageable memory and a launch to gather the view costs took
+  // 39 us of a simplex step's 249
   cudaStream_t s = S(stream);
-  ASC_CUDA(cudaMemcpyAsync(e->d_bone, bone, n * sizeof(int), cudaMemcpyHostToDevice, s));
-  ASC_CUDA(cudaMemcpyAsync(e->d_manip, manip, n * 6 * sizeof(double), cudaMemcpyHostToDevice, s));
-  int rc = engine_launch(e, n, e->d_bone, e->d_manip, e->d_cost, vcost ? e->d_vcost : nullptr, s);
+  const HostIO& io = e->io;
+  memcpy(io.bone, bone, n * sizeof(int));
+  memcpy(io.manip, manip, n * 6 * sizeof(double));
+  int rc = engine_launch(e, n, io.bone, io.manip, io.cost, vcost ? io.vcost : nullptr, s, false, io.error);
   if (rc) return rc;
-  ASC_CUDA(cudaMemcpyAsync(cost, e->d_cost, n * sizeof(double), cudaMemcpyDeviceToHost, s));
-  if (vcost)
-    ASC_CUDA(cudaMemcpyAsync(vcost, e->d_vcost, (size_t)n * e->host.slots * sizeof(double), cudaMemcpyDeviceToHost, s));
-  Counters C;
-  ASC_CUDA(cudaMemcpyAsync(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost, s));
   ASC_CUDA(cudaStreamSynchronize(s));
-  return C.error ? C.error : ASC_OK;
+  memcpy(cost, io.cost, n * sizeof(double));
+  if (vcost) memcpy(vcost, io.vcost, (size_t)n * e->host.slots * sizeof(double));
+  return *io.error ? *io.error : ASC_OK;
 }
 
 ASC_API int asc_engine_debug(asc_engine e, const float** drr, const int** layout)

@@ -1023,14 +1023,80 @@ __device__ __noinline__ float* run_chain(const FilterDev* fl, int nf, int H, flo
   return in;
 }
 
+// Calls f(i, ly, lx) for the tile's pixels, i = ly VT + lx, thread t taking t,
+// t + VNT, ...
+template <class F>
+__device__ __forceinline__ void for_tile(F&& f)
+{
+  int ly = threadIdx.x / VT, lx = threadIdx.x % VT;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < VT * VT; i += VNT) {
+    f(i, ly, lx);
+    lx += VNT % VT;
+    ly += VNT / VT;
+    if (lx >= VT) {
+      lx -= VT;
+      ++ly;
+    }
+  }
+}
+
+// The radiograph crop (RadRenderer_kernels.cu:85-116) over the tile and the
+// chain's halo, four pixels at a time so that sixteen texels are in flight;
+// 0 outside the image and where a pixel maps outside the radiograph.  The
+// texels and the interpolation are bilinear_at's.
+template <class T>
+__device__ __forceinline__ void rad_band(const T* __restrict__ rad, float scale, int W, int Hr, const Region& g,
+                                         int halo, const int* tcx, const float* tax, const int* tcy, const float* tay,
+                                         float* out)
+{
+  for_units(band(g, halo), [&](int ry, int rx) {
+    const int ky = tcy[ry];
+    const bool row = ky != kNoTexel && (g.in || (g.y0 + ry >= 0 && g.y0 + ry < g.h));
+    const float ay = tay[ry];
+    const T *ra = rad + (size_t)min(max(ky, 0), Hr - 1) * W, *rb = rad + (size_t)min(max(ky + 1, 0), Hr - 1) * W;
+    float o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int kx = tcx[rx + i];
+      const bool at = row && kx != kNoTexel && (g.in || (g.x0 + rx + i >= 0 && g.x0 + rx + i < g.w));
+      o[i] = 0.f;
+      if (at) {
+        const int xa = min(max(kx, 0), W - 1), xb = min(max(kx + 1, 0), W - 1);
+        const float ax = tax[rx + i];
+        // rounded before they are used, as image_texel's are
+        const float v00 = __fmul_rn(__ldg(ra + xa), scale), v01 = __fmul_rn(__ldg(ra + xb), scale);
+        const float v10 = __fmul_rn(__ldg(rb + xa), scale), v11 = __fmul_rn(__ldg(rb + xb), scale);
+        const float r0 = fmaf(ax, v01 - v00, v00), r1 = fmaf(ax, v11 - v10, v10);
+        o[i] = 1.0f - fmaf(ay, r1 - r0, r0);
+      }
+    }
+    *reinterpret_cast<float4*>(out + ry * g.P + rx) = make_float4(o[0], o[1], o[2], o[3]);
+  });
+}
+
+// BackgroundRenderer's mask (BackgroundRenderer_kernels.cu:88-120) at a pixel.
+__device__ __noinline__ float background(const ViewDev& V, const IV& r, const double* rcp, int x, int y)
+{
+  int kx, ky;
+  float ax, ay;
+  if (!image_axis(r.vp[0], r.vp[2], x, r.w, rcp[0], V.ipf[0], V.ipf[2], rcp[2], V.bg_w, false, kx, ax) ||
+      !image_axis(r.vp[1], r.vp[3], y, r.h, rcp[1], V.ipf[1], V.ipf[3], rcp[3], V.bg_h, true, ky, ay))
+    return 0.0f;
+  return V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, ax, ky, ay) ? 1.0f : 0.0f;
+}
+
 // One 48 x 48 output tile after another from a queue.  What bounds it is
 // instruction issue (55 %) and, at 24 warps per SM, the barriers between its
 // stages.  On 300 candidates x 2 views of 1024^2 with the four-filter chain:
 // 3.58 ms with one column per unit and the FP64 quotients by division, 2.84
-// here; 64 candidates under SAD at 771 x 645: 1.20 and 0.95.  The last
-// thread grabs the next tile while this one is filtered, and warp 0 alone
-// finishes a tile (its FP64 moments, the view's merge, the item's cost) while
-// the other warps go on to the next.
+// with four columns, 2.63 with the radiograph's texels fetched sixteen at a
+// time and the masked pixels kept by their value instead of a flag; one
+// candidate of two 256^2 views (latency alone: FP64 chains of one warp,
+// round trips to L2, code met for the first time): 61 and 50 us by the moments'
+// fields dealt to lanes.  The last thread grabs the next tile while this one is
+// filtered, and warp 0 alone finishes a tile (its FP64 moments, the view's
+// merge, the item's cost) while the other warps go on to the next.
 __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     k_view(const SceneDev* __restrict__ sc, Bufs b, double* __restrict__ cost, double* __restrict__ view_cost_out)
 {
@@ -1038,6 +1104,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
   __shared__ int s_tile[2], s_k[2];  // this tile's and the next one's
   __shared__ float red[8 * 6 * 2];
   __shared__ double ds[6], dc[3];
+  __shared__ float s_mean[2];
   __shared__ double s_rcp[4];  // 1 / w, 1 / h of the crop; 1 / the image's width and height on the film plane
   __shared__ float wsh[32];
   __shared__ unsigned s_keep[VNT / 32];
@@ -1084,7 +1151,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       const Band d = band(g, V.h_drr);
       for_band(d, [&](int ry, int rx) {
         const bool in = g.in || inside(g, ry, rx);
-        const float* src = in ? drr + (long long)(g.y0 + ry) * r.w + g.x0 + rx : drr;
+        const float* src = in ? drr + (long long)(g.y0 + ry) * g.w + g.x0 + rx : drr;
         const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + ry * P + rx);
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 4 : 0)
                      : "memory");
@@ -1097,12 +1164,11 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         s_rcp[threadIdx.x] = reciprocal(v);
       }
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      __syncthreads();
       if (grabs) {  // for after this tile's last barrier
         s_tile[turn ^ 1] = next;
         s_k[turn ^ 1] = next_k;
       }
-      bool nz = false;
+      bool nz = false;  // of the words that this thread copied
       for_band(d, [&](int ry, int rx) { nz |= buf[ry * P + rx] != 0.f; });
       live = __syncthreads_or(nz);
     }
@@ -1134,20 +1200,16 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       // ---- radiograph crop and its chain
       float* gres;
       {
-        for_band(band(g, V.h_rad), [&](int ry, int rx) {
-          float val = 0.f;
-          const int kx = tcx[rx], ky = tcy[ry];
-          if ((g.in || inside(g, ry, rx)) && kx != kNoTexel && ky != kNoTexel)
-            val = 1.0f - bilinear_at(V.rad, V.rad_bps, V.rad_w, V.rad_h, kx, tax[rx], ky, tay[ry]);
-          buf[ry * P + rx] = val;
-        });
+        if (V.rad_bps == 16)
+          rad_band((const unsigned short*)V.rad, 1.0f / 65535.0f, V.rad_w, V.rad_h, g, V.h_rad, tcx, tax, tcy, tay, buf);
+        else
+          rad_band((const unsigned char*)V.rad, 1.0f / 255.0f, V.rad_w, V.rad_h, g, V.h_rad, tcx, tax, tcy, tay, buf);
         __syncthreads();
         gres = run_chain(V.frad, V.n_rad, V.h_rad, buf, size, wsh, g) + H * P + EX;
       }
       // ---- masks and moments (Tracker.cpp:744-770), two passes over the
-      // tile: f = DRR * mask over fdrr, g = rad * mask over the chain result,
-      // the m > 0.5 flags in the free blur buffer
-      const unsigned n = (unsigned)r.w * (unsigned)r.h;
+      // tile: f = DRR * mask over fdrr, g = rad * mask over the chain result
+      const unsigned n = (unsigned)g.w * (unsigned)g.h;
       const bool tree = sc->coverage == ASC_SUM_TREE && tree_needed(n);  // else every pixel counts
       int shift = 0;
       if (tree) {
@@ -1155,63 +1217,51 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         __syncthreads();
       }
       const bool sad = sc->cf_model != 0;
-      float* flag = buf + 2 * size;
       // per tile: the pixels with mask 1 and their sums of f and g.  The
       // mask is 0 or 1 and f, g are 0 where it is 0, so these are also the
-      // covered pixels' sums of mask, f and g.  Plain FP32 suffices for them:
-      // an error in a tile's mean moves the centred moments only at second
-      // order; the products are the sums that need compensating.
+      // covered pixels' sums of mask, f and g, and a pixel with f != 0 is one
+      // under the mask.  Plain FP32 suffices for them: an error in a tile's
+      // mean moves the centred moments only at second order; the products are
+      // the sums that need compensating.
+      const bool has_bg = V.bg && V.bg_thr >= 0.f;
+      float2* fg = b.fg + r.pix;
       float s[3] = {0.f, 0.f, 0.f};
-      for (int i = threadIdx.x; i < VT * VT; i += VNT) {
-        const int ly = i / VT, lx = i % VT, x = tx0 + lx, y = ty0 + ly;
-        const int gi = ly * P + lx;
-        float f = 0.f, gm = 0.f, fl = 0.f;
-        if (x < r.w && y < r.h && (!tree || tree_kept(s_keep, (unsigned)(y * r.w + x), shift))) {
-          float d = fdrr[i], gg = gres[gi];
-          float bg = 1.0f;
-          if (V.bg && V.bg_thr >= 0.f) {
-            int kx, ky;
-            float ax, ay;
-            bg = image_axis(r.vp[0], r.vp[2], x, r.w, s_rcp[0], V.ipf[0], V.ipf[2], s_rcp[2], V.bg_w, false, kx, ax) &&
-                     image_axis(r.vp[1], r.vp[3], y, r.h, s_rcp[1], V.ipf[1], V.ipf[3], s_rcp[3], V.bg_h, true, ky, ay)
-                   ? (V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, ax, ky, ay) ? 1.0f : 0.0f)
-                   : 0.0f;
-          }
-          float m = bg * (d != 0.0f ? 1.0f : 0.0f);
+      for_tile([&](int i, int ly, int lx) {
+        const int x = tx0 + lx, y = ty0 + ly;
+        float f = 0.f, gm = 0.f;
+        const bool at = x < g.w && y < g.h;
+        if (at && (!tree || tree_kept(s_keep, (unsigned)(y * g.w + x), shift))) {
+          const float d = fdrr[i], gg = gres[ly * P + lx];
+          float m = d != 0.0f ? 1.0f : 0.0f;
+          if (has_bg) m *= background(V, r, s_rcp, x, y);
           f = d * m;
           gm = gg * m;
           if (m > 0.5f) {
-            fl = 1.f;
             s[0] += 1.f;
             s[1] += f;
             s[2] += gm;
           }
         }
         fdrr[i] = f;
-        gres[gi] = gm;
-        flag[i] = fl;
+        gres[ly * P + lx] = gm;
         // SAD needs the view's global means first: keep f and g for k_sad
-        if (sad && x < r.w && y < r.h) b.fg[r.pix + (long long)y * r.w + x] = make_float2(f, gm);
-      }
-      // the sums (ds[3 ..]), and the tile's FP32 centres from them
-      block_sum_f<3>(s, red, ds + 3);
-      if (threadIdx.x < 3) {
-        const double cnt = ds[3], mine = ds[3 + threadIdx.x];
-        ds[threadIdx.x] = mine;
-        red[threadIdx.x] = cnt > 0 ? (float)(mine / cnt) : 0.f;
-      }
-      __syncthreads();
-      mf = red[1];
-      mg = red[2];
+        if (sad && at) fg[(long long)y * g.w + x] = make_float2(f, gm);
+      });
+      // the sums, and the tile's FP32 centres from them
+      block_means(s, red, ds + 3, s_mean);
+      mf = s_mean[0];
+      mg = s_mean[1];
       DFs c[3] = {};  // compensated co-moments about (mf, mg)
-      for (int i = threadIdx.x; i < VT * VT && !sad; i += VNT)
-        if (flag[i] != 0.f) {
-          const int ly = i / VT, lx = i % VT;
-          float a = fdrr[i] - mf, bb = gres[ly * P + lx] - mg;
+      if (!sad)
+        for_tile([&](int i, int ly, int lx) {
+          const float f = fdrr[i];
+          if (f == 0.f) return;
+          const float a = f - mf, bb = gres[ly * P + lx] - mg;
           dfs_add_prod(c[0], a, a);
           dfs_add_prod(c[1], bb, bb);
           dfs_add_prod(c[2], a, bb);
-        }
+        });
+      if (threadIdx.x < 3) ds[threadIdx.x] = ds[3 + threadIdx.x];  // read past the next barrier
       block_sum_dfs<3>(c, red, dc);
     }
     if (threadIdx.x >= 32) continue;
@@ -1219,10 +1269,13 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     // tiles, the last view of an item sums the view costs
     const int lane = threadIdx.x, nt = r.ftx * r.fty;
     bool last = false;
+    if (live)
+      tile_moments(ds, dc, mf, mg, b.part + tile);
+    else if (lane < 9)
+      ((double*)(b.part + tile))[lane] = 0.0;  // zeros add nothing
+    __threadfence();
+    __syncwarp();
     if (lane == 0) {
-      const double zero[6] = {0, 0, 0, 0, 0, 0};
-      b.part[tile] = live ? tile_moments(ds, dc, mf, mg) : tile_moments(zero, zero, 0.f, 0.f);  // zeros add nothing
-      __threadfence();
       last = atomicAdd(&b.ivt[k], 1u) == (unsigned)nt - 1;
     }
     if (!__shfl_sync(FULL_WARP, (int)last, 0)) continue;

@@ -211,50 +211,80 @@ struct Moments {
 
 // The moments of `nb` blocks or tiles, merged in FP64 by one warp: the exact
 // mean from theirs, then each one's co-moments moved to it (C + n (mean - M)
-// (mean' - M')), two sweeps with two divisions where merging them pairwise
-// (Chan et al.) took eight levels of three, at ~70 cycles an operation.
+// (mean' - M')), where merging them pairwise (Chan et al.) took eight levels of
+// three divisions.  It runs once per result, so its time is latency: of loads
+// of what other SMs have just written (~1000 cycles), of dependent FP64
+// operations (~70) and of its code's first fetch.  So a lane loads two
+// partials' nine fields at once and keeps them for the second sweep, the sums
+// of a sweep share a butterfly, and the two means a division.  On one
+// candidate of two 256^2 views (36 tiles each) k_view took 50 us with it, 63
+// with a lane per field and group of partials, 61 with a load per use.
 __device__ __forceinline__ double warp_sum_d(double v)
 {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&v)[N])
+{
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+}
 __device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
 {
+  constexpr int KEEP = 2;
   const int lane = threadIdx.x & 31;
-  Moments a = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = lane; i < nb; i += 32) {
-    const Moments* p = part + i;
-    const double n = __ldcg(&p->n);
-    a.sm += __ldcg(&p->sm);
-    a.sf += __ldcg(&p->sf);
-    a.sg += __ldcg(&p->sg);
-    a.n += n;
-    a.mf += n * __ldcg(&p->mf);
-    a.mg += n * __ldcg(&p->mg);
+  const double* p = (const double*)part;  // nine fields: sm sf sg n mf mg cff cgg cfg
+  double kept[KEEP][9];
+#pragma unroll
+  for (int t = 0; t < KEEP; ++t)
+#pragma unroll
+    for (int f = 0; f < 9; ++f) kept[t][f] = lane + 32 * t < nb ? __ldcg(p + 9 * (lane + 32 * t) + f) : 0.0;
+  double a[6] = {};  // sm, sf, sg, n and the sums of n mf, n mg
+  const auto first = [&](const double* v) {
+#pragma unroll
+    for (int f = 0; f < 4; ++f) a[f] += v[f];
+    a[4] = fma(v[3], v[4], a[4]);
+    a[5] = fma(v[3], v[5], a[5]);
+  };
+#pragma unroll
+  for (int t = 0; t < KEEP; ++t) first(kept[t]);
+#pragma unroll 1
+  for (int i = lane + 32 * KEEP; i < nb; i += 32) {
+    double v[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) v[f] = __ldcg(p + 9 * i + f);
+    first(v);
   }
-  a.n = warp_sum_d(a.n);
-  a.sm = warp_sum_d(a.sm);
-  a.sf = warp_sum_d(a.sf);
-  a.sg = warp_sum_d(a.sg);
-  a.mf = warp_sum_d(a.mf);
-  a.mg = warp_sum_d(a.mg);
-  if (!(a.n > 0)) return a;
-  a.mf /= a.n;
-  a.mg /= a.n;
-  for (int i = lane; i < nb; i += 32) {
-    const Moments* p = part + i;
-    const double n = __ldcg(&p->n), df = __ldcg(&p->mf) - a.mf, dg = __ldcg(&p->mg) - a.mg;
-    if (n > 0) {
-      a.cff += __ldcg(&p->cff) + n * df * df;
-      a.cgg += __ldcg(&p->cgg) + n * dg * dg;
-      a.cfg += __ldcg(&p->cfg) + n * df * dg;
+  warp_sums(a);
+  double c[3] = {}, mf = 0.0, mg = 0.0;
+  const auto second = [&](const double* v) {
+    if (!(v[3] > 0)) return;
+    const double df = v[4] - mf, dg = v[5] - mg;
+    c[0] += fma(v[3] * df, df, v[6]);
+    c[1] += fma(v[3] * dg, dg, v[7]);
+    c[2] += fma(v[3] * df, dg, v[8]);
+  };
+  if (a[3] > 0) {
+    const double mean = (lane == 0 ? a[4] : a[5]) / a[3];
+    mf = __shfl_sync(0xffffffffu, mean, 0);
+    mg = __shfl_sync(0xffffffffu, mean, 1);
+#pragma unroll
+    for (int t = 0; t < KEEP; ++t) second(kept[t]);
+#pragma unroll 1
+    for (int i = lane + 32 * KEEP; i < nb; i += 32) {
+      double v[9];
+#pragma unroll
+      for (int f = 3; f < 9; ++f) v[f] = __ldcg(p + 9 * i + f);
+      second(v);
     }
+    warp_sums(c);
   }
-  a.cff = warp_sum_d(a.cff);
-  a.cgg = warp_sum_d(a.cgg);
-  a.cfg = warp_sum_d(a.cfg);
-  return a;
+  return Moments{a[0], a[1], a[2], a[3], mf, mg, c[0], c[1], c[2]};
 }
+static_assert(sizeof(Moments) == 9 * sizeof(double), "nine fields");
 
 // ---- compensated FP32 sums ----
 // A double-float accumulator, value = h + l: each addition is Knuth's
@@ -289,14 +319,15 @@ __device__ __forceinline__ void dfs_merge(DFs& a, const DFs& b)
   a.l = __fadd_rn(a.l, b.l);
 }
 
-// Block-wide sums of N compensated accumulators: a TwoSum butterfly within
-// each warp, then the warps' pairs added in FP64 by N threads.  red: 2 N
-// floats per warp of the block; out (shared): the N sums, visible to every
-// thread on return.
+// Block-wide sums of N compensated accumulators of a block of 256 threads: a
+// TwoSum butterfly within each warp, then the warps' pairs added in FP64 by 8
+// lanes per sum.  red: 2 N floats per warp of the block; out (shared): the N
+// sums, visible to every thread on return.
 template <int N>
 __device__ __forceinline__ void block_sum_dfs(DFs (&v)[N], float* red, double* out)
 {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  static_assert(N <= 4, "8 lanes per sum");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < N; ++k)
 #pragma unroll
@@ -312,34 +343,39 @@ __device__ __forceinline__ void block_sum_dfs(DFs (&v)[N], float* red, double* o
       red[(warp * N + k) * 2 + 1] = v[k].l;
     }
   __syncthreads();
-  if (threadIdx.x < N) {
-    double t = 0.0;
-    for (int j = 0; j < nw; ++j) t += (double)red[(j * N + threadIdx.x) * 2] + (double)red[(j * N + threadIdx.x) * 2 + 1];
-    out[threadIdx.x] = t;
+  if (warp == 0) {
+    const int k = min(lane >> 3, N - 1), j = lane & 7;
+    double t = (double)red[(j * N + k) * 2] + (double)red[(j * N + k) * 2 + 1];
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (j == 0 && lane < 8 * N) out[lane >> 3] = t;
   }
   __syncthreads();
 }
 
-// Block-wide FP32 sums of N values (a shuffle butterfly per warp, the warps'
-// sums added in FP64 by N threads); out (shared) is visible to every thread
-// on return.  red: N floats per warp.
-template <int N>
-__device__ __forceinline__ void block_sum_f(float (&v)[N], float* red, double* out)
+// Block-wide FP32 sums of a count and two values of a block of 256 threads (a
+// shuffle butterfly per warp, the warps' sums added in FP64), and the two
+// values' means in FP32 (0 without a count); out (3 sums) and mean (2),
+// shared, are visible to every thread on return.  red: 3 floats per warp.
+__device__ __forceinline__ void block_means(float (&v)[3], float* red, double* out, float* mean)
 {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < N; ++k)
+  for (int k = 0; k < 3; ++k)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
   __syncthreads();
   if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < N; ++k) red[warp * N + k] = v[k];
+    for (int k = 0; k < 3; ++k) red[warp * 3 + k] = v[k];
   __syncthreads();
-  if (threadIdx.x < N) {
-    double t = 0.0;
-    for (int j = 0; j < nw; ++j) t += (double)red[j * N + threadIdx.x];
-    out[threadIdx.x] = t;
+  if (warp == 0) {
+    const int k = min(lane >> 3, 2);
+    double t = (double)red[(lane & 7) * 3 + k];
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const double n = __shfl_sync(0xffffffffu, t, 0);
+    const double q = n > 0 ? t / n : 0.0;
+    if (lane == 0 || lane == 8 || lane == 16) out[k] = t;
+    if (lane == 8 || lane == 16) mean[k - 1] = (float)q;
   }
   __syncthreads();
 }
@@ -350,21 +386,21 @@ __device__ __forceinline__ void block_sum_f(float (&v)[N], float* red, double* o
 // exact tile means replace the centres, with the co-moments moved to them
 // (C - n (mean - centre)(mean' - centre')), so the FP64 merge sees exact
 // centred moments whatever the centres' rounding.
-__device__ __forceinline__ Moments tile_moments(const double* s, const double* c, float cf, float cg)
+// By a warp, a lane per field of *out (the quotients side by side, one store).
+__device__ __forceinline__ void tile_moments(const double* s, const double* c, float cf, float cg, Moments* out)
 {
-  Moments p = {s[0], s[1], s[2], s[3], 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (s[3] > 0) {
-    const double n = s[3], mf = s[4] / n, mg = s[5] / n, df = mf - (double)cf, dg = mg - (double)cg;
-    p.mf = mf;
-    p.mg = mg;
-    // sums of squares about the mean: rounding must not leave them below 0
-    // (a tile of equal values gives C = n (mean - centre)^2 up to rounding)
-    const double ff = c[0] - n * df * df, gg = c[1] - n * dg * dg;
-    p.cff = ff < 0.0 ? 0.0 : ff;
-    p.cgg = gg < 0.0 ? 0.0 : gg;
-    p.cfg = c[2] - n * df * dg;
-  }
-  return p;
+  const int lane = threadIdx.x & 31;
+  const double n = s[3];
+  const double mean = n > 0 ? s[4 + (lane & 1)] / n : 0.0;
+  const double off = mean - (double)(lane == 0 ? cf : cg);
+  const double df = __shfl_sync(0xffffffffu, off, 0), dg = __shfl_sync(0xffffffffu, off, 1);
+  // sums of squares about the mean: rounding must not leave them below 0
+  // (a tile of equal values gives C = n (mean - centre)^2 up to rounding)
+  const int q = min(max(lane - 6, 0), 2);
+  double moved = c[q] - n * (q == 1 ? dg : df) * (q == 0 ? df : dg);
+  if ((q < 2 && moved < 0.0) || !(n > 0)) moved = 0.0;
+  const double m = __shfl_sync(0xffffffffu, mean, lane == 5 ? 1 : 0);
+  if (lane < 9) ((double*)out)[lane] = lane < 4 ? s[lane] : (lane < 6 ? m : moved);
 }
 
 // gpu::ncc's result from the merged moments (Ncc_kernels.cu:116-134):

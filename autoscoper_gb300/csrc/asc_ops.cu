@@ -519,9 +519,10 @@ __global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const f
   wide_sum_dfs<3>(c, red, dc);
   if (threadIdx.x >= 32) return;
   bool last = false;
+  tile_moments(ds, dc, mf, mg, sc.part + blockIdx.x);
+  __threadfence();
+  __syncwarp();
   if (threadIdx.x == 0) {
-    sc.part[blockIdx.x] = tile_moments(ds, dc, mf, mg);
-    __threadfence();
     last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
   }
   if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;

@@ -624,6 +624,7 @@ __global__ void __launch_bounds__(NRAY, ASC_RAY_MINBLOCKS) k_ray(const SceneDev*
     if (valid) *out = flagged ? -1.0f : fminf(fmaxf(d * B.scale[r.slot], 0.f), 1.f);
     if (__any_sync(FULL_WARP, flagged) && lane == 0) b.fixb[atomicAdd(&b.C->nfixb, 1)] = id;
   }
+  for (int o = 16; o > 0; o >>= 1) marched += __shfl_xor_sync(FULL_WARP, marched, o);
   if (lane == 0 && slots) {
     atomicAdd(&b.C->marched, marched);
     atomicAdd(&b.C->slots, slots);

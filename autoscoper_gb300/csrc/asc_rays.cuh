@@ -21,8 +21,10 @@
 // room for), so sorting a block's segments by length, with its barriers, costs
 // more than the idle lanes do (12.6 ms against 12.2 on the batch below).
 // k_ray over 300 candidates x 2 views of 1024^2 (three bones of up to 4.8 M
-// voxels): 16.5 ms with the walk, 12.2 here (15.7 G and 11.0 G warp
-// instructions); 100 candidates of a 128^3 bone at 512^2: 2.55 and 1.44 ms.
+// voxels): 16.5 ms with the walk, 12.2 with beams (15.7 G and 11.0 G warp
+// instructions), 11.8 with the sample loop's unpacking split over two units
+// and no clamp in it (march_block); 100 candidates of a 128^3 bone at 512^2:
+// 2.55, 1.44 and 1.42 ms.
 #pragma once
 
 #include "asc_internal.cuh"
@@ -167,8 +169,10 @@ __device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* 
 }
 
 // The segments of this lane's ray (K samples; 0: none), marched side by side
-// with the warp's other lanes.  Returns their sum in raw units: NaN when a
-// sample fell in the cutoff's band.
+// with the warp's other lanes.  tf: RaySetup::tf, negative for a ray that is
+// not ray_inside().  Returns their sum in raw units: NaN when a sample fell in
+// the cutoff's band.  marched: this lane's samples; slots: what the warp's
+// lanes had room for.
 template <int STORE, int PAIRS, class Slots>
 __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* __restrict__ clr, const Slots& S,
                                             int K, float tf, const Beam& b, float4 band, const Cutoff& cut,
@@ -179,7 +183,7 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
   df total{0.f, 0.f};  // NaN once a segment met the cutoff's band
   for (;;) {
     int kb, js, je, len = 0;
-    if (next_segment(V, clr, S, K, tf, b, run, kb, js, je)) {
+    if (next_segment(V, clr, S, K, fabsf(tf), b, run, kb, js, je)) {
       RaySetup r;
       const float4 q0 = S.q[0][threadIdx.x], q1 = S.q[1][threadIdx.x], q2 = S.q[2][threadIdx.x];
       r.X = df{q0.x, q0.y};
@@ -190,7 +194,8 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
       r.dZ = df{q2.z, q2.w};
       // this ray's band: raw - t0, hi0 + t0 and t1 (cutoff_bounds)
       const float D = fabsf(q1.z) + fabsf(q2.x) + fabsf(q2.z);
-      const float p = march_block<STORE, false, PAIRS>(V, r, kb, js, je, fmaf(-band.z, D, band.x), fmaf(band.z, D, band.y), cut);
+      const float p = march_block<STORE, false, PAIRS>(V, r, kb, js, je, fmaf(-band.z, D, band.x),
+                                                       fmaf(band.z, D, band.y), cut, tf > 0.f);
       if (block_flagged(p))
         total.h = __int_as_float(0x7fffffff);  // NaN stays NaN through add_block
       else
@@ -199,7 +204,7 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
     }
     const unsigned most = __reduce_max_sync(FULL_WARP, (unsigned)len);
     if (most == 0) break;
-    marched += __reduce_add_sync(FULL_WARP, (unsigned)len);
+    marched += (unsigned)len;
     slots += 32u * most;
   }
   return total.h + total.l;
@@ -221,7 +226,7 @@ __device__ __forceinline__ float ray_beam(const DevVolume& V, const RayScene& s,
       S.q[1][threadIdx.x] = make_float4(r.Z.h, r.Z.l, r.dX.h, r.dX.l);
       S.q[2][threadIdx.x] = make_float4(r.dY.h, r.dY.l, r.dZ.h, r.dZ.l);
       K = r.K;
-      tf = r.tf;
+      tf = ray_inside(V, r) ? r.tf : -r.tf;
     }
   }
   if (V.storage == ASC_STORE_F32) return march_beam<ASC_STORE_F32, PAIRS>(V, s.clr, S, K, tf, b, band, cut, marched, slots);

@@ -257,7 +257,7 @@ __device__ __forceinline__ float march_pass(const DevVolume& V, const uint8_t* _
     ia = t.ia[i];
     c = t.c[i];
   }, s, [&](int kb, int js, int je) {
-    const float p = march_block<STORE, EXACT>(V, r, kb, js, je, lo, hi, cut);
+    const float p = march_block<STORE, EXACT>(V, r, kb, js, je, lo, hi, cut, ray_inside(V, r));
     if (!EXACT && block_flagged(p))
       fl = true;
     else

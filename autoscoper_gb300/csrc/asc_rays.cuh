@@ -23,8 +23,9 @@
 // k_ray over 300 candidates x 2 views of 1024^2 (three bones of up to 4.8 M
 // voxels): 16.5 ms with the walk, 12.2 with beams (15.7 G and 11.0 G warp
 // instructions), 11.8 with the sample loop's unpacking split over two units
-// and no clamp in it (march_block); 100 candidates of a 128^3 bone at 512^2:
-// 2.55, 1.44 and 1.42 ms.
+// and no clamp in it (march_block), 11.3 with the warp met again before each
+// march (march_beam); 100 candidates of a 128^3 bone at 512^2: 2.55, 1.44,
+// 1.42 and 1.37 ms.
 #pragma once
 
 #include "asc_internal.cuh"
@@ -121,8 +122,7 @@ __device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* 
                                              int K, float tf, const Beam& b, RunState& s, int& kb, int& js, int& je)
 {
   for (;;) {
-    if (s.k > s.ke) {
-      if (!s.mask) break;
+    while (s.k > s.ke && s.mask) {
       // the run of intervals farthest from the camera (samples count from the far side)
       const int i1 = 63 - __clzll((long long)s.mask);
       const unsigned long long above = ~(s.mask << (63 - i1));
@@ -149,8 +149,8 @@ __device__ __forceinline__ bool next_segment(const DevVolume& V, const uint8_t* 
           if (f + l == 0) break;
         }
       }
-      continue;
     }
+    if (s.k > s.ke) break;
     const int bb = (int)((unsigned)s.k / REBASE), hi = min(s.ke, bb * REBASE + REBASE - 1);
     if (s.pf >= 0 && s.pb != bb) break;
     if (s.pf < 0) {
@@ -182,8 +182,22 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
   if (K <= 0) run.mask = 0;
   df total{0.f, 0.f};  // NaN once a segment met the cutoff's band
   for (;;) {
-    int kb, js, je, len = 0;
-    if (next_segment(V, clr, S, K, fabsf(tf), b, run, kb, js, je)) {
+    // A segment or an empty one in the same registers, and what depends on it
+    // after the warp has met again: with the march under next_segment's own
+    // result the compiler ran all that follows twice, for the lanes that had
+    // a segment and for the others (k_ray 11.81 ms against 11.31 here).
+    int kb = 0, js = 0, je = -1;
+    {
+      int a, f, l;
+      if (next_segment(V, clr, S, K, fabsf(tf), b, run, a, f, l)) {
+        kb = a;
+        js = f;
+        je = l;
+      }
+    }
+    const int len = je - js + 1;
+    float p = 0.f;
+    if (len > 0) {
       RaySetup r;
       const float4 q0 = S.q[0][threadIdx.x], q1 = S.q[1][threadIdx.x], q2 = S.q[2][threadIdx.x];
       r.X = df{q0.x, q0.y};
@@ -194,14 +208,13 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
       r.dZ = df{q2.z, q2.w};
       // this ray's band: raw - t0, hi0 + t0 and t1 (cutoff_bounds)
       const float D = fabsf(q1.z) + fabsf(q2.x) + fabsf(q2.z);
-      const float p = march_block<STORE, false, PAIRS>(V, r, kb, js, je, fmaf(-band.z, D, band.x),
-                                                       fmaf(band.z, D, band.y), cut, tf > 0.f);
-      if (block_flagged(p))
-        total.h = __int_as_float(0x7fffffff);  // NaN stays NaN through add_block
-      else
-        add_block(total, p);
-      len = je - js + 1;
+      p = march_block<STORE, false, PAIRS>(V, r, kb, js, je, fmaf(-band.z, D, band.x), fmaf(band.z, D, band.y), cut,
+                                           tf > 0.f);
     }
+    if (block_flagged(p))
+      total.h = __int_as_float(0x7fffffff);  // NaN stays NaN through add_block
+    else
+      add_block(total, p);
     const unsigned most = __reduce_max_sync(FULL_WARP, (unsigned)len);
     if (most == 0) break;
     marched += (unsigned)len;

@@ -4,7 +4,7 @@ An engine evaluation launches the ray cast (persistent blocks per SM, and
 the ray block each warp takes in a 16 x 16 ray tile) and the fused filter /
 NCC kernel (persistent blocks per SM).  The best shapes depend on the
 workload: crop sizes (render size, magnification), volume sizes (how long a
-ray marches, how much of a tile's work is the walk) and the number of views.
+ray marches, how many beams meet a bone) and the number of views.
 For each workload class this module times every candidate shape on that
 workload's own candidate batch with CUDA events (the engine's phase timers),
 keeps the fastest, and writes the table that asc_engine_create reads

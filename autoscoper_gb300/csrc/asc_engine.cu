@@ -1088,7 +1088,7 @@ __device__ __noinline__ float background(const ViewDev& V, const IV& r, const do
 }
 
 // One 48 x 48 output tile after another from a queue.  What bounds it is
-// instruction issue (55 %) and, at 24 warps per SM, the barriers between its
+// instruction issue (60 %) and, at 24 warps per SM, the barriers between its
 // stages.  On 300 candidates x 2 views of 1024^2 with the four-filter chain:
 // 3.58 ms with one column per unit and the FP64 quotients by division, 2.84
 // with four columns, 2.63 with the radiograph's texels fetched sixteen at a

@@ -1076,15 +1076,39 @@ __device__ __forceinline__ void rad_band(const T* __restrict__ rad, float scale,
   });
 }
 
-// BackgroundRenderer's mask (BackgroundRenderer_kernels.cu:88-120) at a pixel.
-__device__ __noinline__ float background(const ViewDev& V, const IV& r, const double* rcp, int x, int y)
+// BackgroundRenderer's mask (BackgroundRenderer_kernels.cu:88-120) over the
+// tile's DRR: 0 where the background image lies below its threshold.  The
+// film-plane mapping once per column and row, in FP64, as the radiograph's and
+// in its tables (free after its chain's barriers): per pixel it was half of
+// the kernel (64 candidates under SAD at 771 x 645 with a background: 980 us
+// with k_sad, 447 here).  A call: inlined, tiles without a background lost 2 %
+// to spilled registers.
+__device__ __noinline__ void background_mask(const ViewDev& V, const IV& r, const double* rcp, Region g, float* fdrr)
 {
-  int kx, ky;
-  float ax, ay;
-  if (!image_axis(r.vp[0], r.vp[2], x, r.w, rcp[0], V.ipf[0], V.ipf[2], rcp[2], V.bg_w, false, kx, ax) ||
-      !image_axis(r.vp[1], r.vp[3], y, r.h, rcp[1], V.ipf[1], V.ipf[3], rcp[3], V.bg_h, true, ky, ay))
-    return 0.0f;
-  return V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, ax, ky, ay) ? 1.0f : 0.0f;
+  extern __shared__ float smem[];
+  int* tcx = (int*)(smem + view_tail_floats(g.EY));
+  float* tax = (float*)(tcx + VT);
+  int* tcy = (int*)(tax + VT);
+  float* tay = (float*)(tcy + VT);
+  const int x0 = g.x0 + g.EX, y0 = g.y0 + g.EY;
+  for (int i = threadIdx.x; i < 2 * VT; i += VNT) {
+    const bool row = i >= VT;
+    const int j = row ? i - VT : i;
+    int q;
+    float a = 0.f;
+    const bool ok = row ? image_axis(r.vp[1], r.vp[3], y0 + j, r.h, rcp[1], V.ipf[1], V.ipf[3], rcp[3], V.bg_h, true, q, a)
+                        : image_axis(r.vp[0], r.vp[2], x0 + j, r.w, rcp[0], V.ipf[0], V.ipf[2], rcp[2], V.bg_w, false, q, a);
+    (row ? tcy : tcx)[j] = ok ? q : kNoTexel;
+    (row ? tay : tax)[j] = a;
+  }
+  __syncthreads();
+  // the words that this thread's pass over the masks reads
+  for_tile([&](int i, int ly, int lx) {
+    const int kx = tcx[lx], ky = tcy[ly];
+    if (fdrr[i] != 0.0f && !(kx != kNoTexel && ky != kNoTexel &&
+                             V.bg_thr <= bilinear_at(V.bg, 32, V.bg_w, V.bg_h, kx, tax[lx], ky, tay[ly])))
+      fdrr[i] = 0.0f;
+  });
 }
 
 // One 48 x 48 output tile after another from a queue.  What bounds it is
@@ -1224,7 +1248,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
       // under the mask.  Plain FP32 suffices for them: an error in a tile's
       // mean moves the centred moments only at second order; the products are
       // the sums that need compensating.
-      const bool has_bg = V.bg && V.bg_thr >= 0.f;
+      if (V.bg && V.bg_thr >= 0.f) background_mask(V, r, s_rcp, g, fdrr);
       float2* fg = b.fg + r.pix;
       float s[3] = {0.f, 0.f, 0.f};
       for_tile([&](int i, int ly, int lx) {
@@ -1233,8 +1257,7 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
         const bool at = x < g.w && y < g.h;
         if (at && (!tree || tree_kept(s_keep, (unsigned)(y * g.w + x), shift))) {
           const float d = fdrr[i], gg = gres[ly * P + lx];
-          float m = d != 0.0f ? 1.0f : 0.0f;
-          if (has_bg) m *= background(V, r, s_rcp, x, y);
+          const float m = d != 0.0f ? 1.0f : 0.0f;
           f = d * m;
           gm = gg * m;
           if (m > 0.5f) {

@@ -128,11 +128,12 @@ __host__ __device__ __forceinline__ bool image_axis(double v0, double vw, int x,
 }
 
 // a / 9, correctly rounded, by the same correction (a result so small that an
-// underflow could part them is 0 to the contrast filter either way).
+// underflow could part them is 0 to the contrast filter either way).  An
+// infinity, whose remainder is NaN, is its own quotient.
 __device__ __forceinline__ float ninth(float a)
 {
-  const float r = 1.0f / 9.0f, q = __fmul_rn(a, r);
-  return fmaf(fmaf(-9.0f, q, a), r, q);
+  const float r = 1.0f / 9.0f, q = __fmul_rn(a, r), e = fmaf(-9.0f, q, a);
+  return e == e ? fmaf(e, r, q) : q;
 }
 
 // Bilinear read of an 8/16-bit (normalized) or float image at the pair

@@ -1510,6 +1510,18 @@ struct HostIO {
   int *bone = nullptr, *error = nullptr;
 };
 
+// What the captured swarm iteration holds as launch arguments.
+struct SwarmKey {
+  int particles, skip;
+  double w, c1, c2;
+  uint64_t seed;
+  // a NaN setting matches nothing and is captured anew
+  bool operator==(const SwarmKey& o) const
+  {
+    return particles == o.particles && skip == o.skip && w == o.w && c1 == o.c1 && c2 == o.c2 && seed == o.seed;
+  }
+};
+
 struct asc_engine_s {
   SceneDev host;
   SceneDev* dev = nullptr;
@@ -1534,7 +1546,7 @@ struct asc_engine_s {
   int* sw_iter = nullptr;
   int* sw_frozen = nullptr;
   cudaGraphExec_t pso_exec = nullptr;
-  double pso_key[5] = {0, 0, 0, 0, 0};
+  SwarmKey pso_key{};
   cudaStream_t own_stream = nullptr;
   int* d_bone = nullptr;
   double* d_manip = nullptr;
@@ -2172,9 +2184,9 @@ ASC_API int asc_engine_pso_stall(asc_engine e, int np, int n_iter, int max_stall
   k_pso_init<<<gb, tb, 0, s>>>(sw, nb, np, lo, hi, seed);
   cudaError_t err = cudaGetLastError();
   // one iteration = update -> setup -> ray -> view -> best, captured once per
-  // (particles, w, c1, c2, seed) and replayed n_iter times
-  const double key[5] = {(double)np, w, c1, c2, (double)seed};
-  if (!err && (!e->pso_exec || memcmp(key, e->pso_key, sizeof key) != 0)) {
+  // SwarmKey and replayed n_iter times
+  const SwarmKey key{np, g_empty_skip, w, c1, c2, seed};
+  if (!err && (!e->pso_exec || !(key == e->pso_key))) {
     if (e->pso_exec) {
       cudaGraphExecDestroy(e->pso_exec);
       e->pso_exec = nullptr;
@@ -2190,7 +2202,7 @@ ASC_API int asc_engine_pso_stall(asc_engine e, int np, int n_iter, int max_stall
     }
     if (!err) err = cudaGraphInstantiate(&e->pso_exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
-    if (!err) memcpy(e->pso_key, key, sizeof key);
+    if (!err) e->pso_key = key;
   }
   long long scored = 0;
   int it = 0;

@@ -1541,6 +1541,9 @@ struct asc_engine_s {
   }
   bool prof = false;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  // after the last asc_engine_eval on a stream of the caller's: what reads
+  // the counters waits for it (the other evaluations end in a wait)
+  cudaEvent_t done = nullptr;
   // device PSO: swarm state, the captured iteration and a private stream
   double* sw_buf = nullptr;
   int* sw_iter = nullptr;
@@ -1571,6 +1574,7 @@ struct asc_engine_s {
         if (p) cudaFree(p);
     for (cudaEvent_t x : ev)
       if (x) cudaEventDestroy(x);
+    if (done) cudaEventDestroy(done);
     if (pso_exec) cudaGraphExecDestroy(pso_exec);
     if (own_stream) cudaStreamDestroy(own_stream);
   }
@@ -1779,6 +1783,7 @@ ASC_API int asc_engine_create(int n_views, const asc_view_desc* views, int n_bon
     io.bone = (int*)(io.vcost + n_iv);
     io.error = io.bone + max_items;
   }
+  if (!err) err = cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming);
   const size_t npix = (size_t)rw * rh;
   if (!err) err = e->alloc(e->p_drr, npix);
   if (!err) err = e->alloc(e->p_rad, npix);
@@ -2065,12 +2070,19 @@ ASC_API int asc_engine_profile(asc_engine e, int enable)
   return ASC_OK;
 }
 
-// The last evaluation's counters, its samples counted here.
-static int read_counters(asc_engine e, Counters& C)
+// The last evaluation's counters, its samples counted here if they are asked
+// for.  The evaluation may be on a stream that nothing orders before the
+// default stream, so its event is waited for; and two callers would count into
+// one word, so one at a time.
+static int read_counters(asc_engine e, Counters& C, bool samples)
 {
-  ASC_CUDA(cudaMemset(&e->b.C->samples, 0, sizeof C.samples));
-  k_count_samples<<<e->sms * 8, NRAY>>>(e->b);
-  ASC_LAUNCH_CHECK();
+  ASC_CUDA(cudaEventSynchronize(e->done));
+  Gate g(device_gate());
+  if (samples) {
+    ASC_CUDA(cudaMemset(&e->b.C->samples, 0, sizeof C.samples));
+    k_count_samples<<<e->sms * 8, NRAY>>>(e->b);
+    ASC_LAUNCH_CHECK();
+  }
   ASC_CUDA(cudaMemcpy(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost));
   return ASC_OK;
 }
@@ -2083,8 +2095,9 @@ ASC_API int asc_engine_stats(asc_engine e, float ms[3], unsigned long long* samp
     ASC_CUDA(cudaEventSynchronize(e->ev[3]));
     for (int i = 0; i < 3; ++i) ASC_CUDA(cudaEventElapsedTime(&ms[i], e->ev[i], e->ev[i + 1]));
   }
+  if (!samples && !pixels) return ASC_OK;
   Counters C;
-  int rc = read_counters(e, C);
+  int rc = read_counters(e, C, samples != nullptr);
   if (rc) return rc;
   if (samples) *samples = C.samples;
   if (pixels) *pixels = C.pixels;
@@ -2095,7 +2108,8 @@ ASC_API int asc_engine_exact_rays(asc_engine e, int* n)
 {
   if (!e || !n) return ASC_ERR_ARG;
   Counters C;
-  ASC_CUDA(cudaMemcpy(&C, e->b.C, sizeof C, cudaMemcpyDeviceToHost));
+  int rc = read_counters(e, C, false);
+  if (rc) return rc;
   *n = C.nfix;
   return ASC_OK;
 }
@@ -2104,7 +2118,7 @@ ASC_API int asc_engine_counters(asc_engine e, unsigned long long out[4])
 {
   if (!e || !out) return ASC_ERR_ARG;
   Counters C;
-  int rc = read_counters(e, C);
+  int rc = read_counters(e, C, true);
   if (rc) return rc;
   out[0] = C.samples;
   out[1] = C.pixels;
@@ -2117,7 +2131,14 @@ ASC_API int asc_engine_eval(asc_engine e, int n, const int* bone, const double* 
                             void* stream)
 {
   if (!e || !bone || !manip || !cost || n < 1 || n > e->max_items) return ASC_ERR_ARG;
-  return engine_launch(e, n, bone, manip, cost, vcost, S(stream));
+  cudaStream_t s = S(stream);
+  int rc = engine_launch(e, n, bone, manip, cost, vcost, s);
+  if (rc || !s) return rc;
+  // a captured evaluation runs when its graph does: no event of this call's
+  cudaStreamCaptureStatus capture;
+  ASC_CUDA(cudaStreamIsCapturing(s, &capture));
+  if (capture == cudaStreamCaptureStatusNone) ASC_CUDA(cudaEventRecord(e->done, s));
+  return ASC_OK;
 }
 
 ASC_API int asc_engine_eval_host(asc_engine e, int n, const int* bone, const double* manip, double* cost,

@@ -319,7 +319,9 @@ int asc_engine_stats(asc_engine e, float ms[3], unsigned long long *samples, uns
  * slots the marching warps occupied (32 x the longest segment of each warp's
  * rays, over the segments it marches side by side); out[2] / out[3] is the
  * SIMT efficiency of the march.  out[0] is counted when it is asked for, from
- * the evaluation's own records. */
+ * the evaluation's own records.  This call, asc_engine_stats and
+ * asc_engine_exact_rays wait for an asc_engine_eval that is still queued; one
+ * that a graph replays is the caller's to wait for. */
 int asc_engine_counters(asc_engine e, unsigned long long out[4]);
 /* Rays of the last evaluation that the ray cast marched a second time: rays
  * with a sample whose FP32 value lay within rounding of the cutoff, whose

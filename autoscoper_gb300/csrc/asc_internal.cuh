@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <vector>
 
 #include "../../include/autoscoper_gb300.h"
 
@@ -44,11 +45,37 @@ using Gate = std::lock_guard<std::recursive_mutex>;
 
 namespace asc {
 
+// The plain ray caster's clearance grid of a volume, built for one raw cutoff
+// at a time and shared by the streams and threads that cast it: every stream
+// waits for the build, and a build for another cutoff waits for every cast that
+// reads the grid it writes over (asc_raycast).  A grid that a captured cast
+// reads is never written over: graphs run when they like.
+struct ClearanceCache {
+  std::mutex mu;
+  uint8_t* grid = nullptr;
+  float cutoff = NAN;           // NaN: not built
+  bool captured = false;        // a graph reads `grid`
+  cudaEvent_t built = nullptr;  // after the build
+  struct Reader {
+    cudaStream_t stream;
+    cudaEvent_t cast;  // after the stream's last cast
+  };
+  static constexpr int MAX_READERS = 4;
+  Reader reader[MAX_READERS] = {};
+  int readers = 0, oldest = 0;
+  std::vector<uint8_t*> kept;  // earlier grids that graphs read
+  ClearanceCache() = default;
+  ClearanceCache(const ClearanceCache&) = delete;
+  ~ClearanceCache();
+  // The grid for `cut`, to be read by the next cast on s; read() after it.
+  int use(const DevVolume& V, float cut, cudaStream_t s, bool capturing);
+  int read(cudaStream_t s, bool capturing);
+};
+
 struct asc_volume_host {
   DevVolume dev;
   uint32_t* pairs;
-  uint8_t* clr;     // clearance grid of the plain ray caster ...
-  float clr_cutoff; // ... for this raw cutoff (NaN = not built)
+  ClearanceCache clr;
   float inv_scale[3], inv_trans[3];
   double trans_center[3];
   float min_value, max_value;

@@ -711,6 +711,94 @@ int build_clearance(const DevVolume& V, float cutoff_raw, uint8_t* clr, cudaStre
 
 // ---------------------------------------------------------------- host side
 
+ClearanceCache::~ClearanceCache()
+{
+  if (grid) cudaFree(grid);
+  for (uint8_t* p : kept) cudaFree(p);
+  if (built) cudaEventDestroy(built);
+  for (Reader& r : reader)
+    if (r.cast) cudaEventDestroy(r.cast);
+}
+
+namespace {
+// While a stream of this thread is captured: lets the thread allocate and
+// work on other streams.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  const bool on;
+  explicit RelaxedCapture(bool capturing) : on(capturing)
+  {
+    if (on) cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  ~RelaxedCapture()
+  {
+    if (on) cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+};
+}  // namespace
+
+int ClearanceCache::use(const DevVolume& V, float cut, cudaStream_t s, bool capturing)
+{
+  RelaxedCapture relaxed(capturing);
+  if (!built) ASC_CUDA(cudaEventCreateWithFlags(&built, cudaEventDisableTiming));
+  if (cutoff == cut) {
+    // a graph may run on any stream, so its grid is complete before it is captured
+    ASC_CUDA(capturing ? cudaEventSynchronize(built) : cudaStreamWaitEvent(s, built));
+    return ASC_OK;
+  }
+  cutoff = NAN;
+  if (captured) {
+    kept.push_back(grid);
+    grid = nullptr;
+    captured = false;
+  }
+  if (!grid) {
+    Gate g(device_gate());
+    readers = 0;
+    ASC_CUDA(cudaMalloc(&grid, clearance_cells(V)));
+  }
+  struct Own {  // what a captured cast reads is built now, not by the graph
+    cudaStream_t s = nullptr;
+    ~Own()
+    {
+      if (s) cudaStreamDestroy(s);
+    }
+  } own;
+  if (capturing) {
+    ASC_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+    s = own.s;
+  }
+  for (int i = 0; i < readers; ++i) ASC_CUDA(cudaStreamWaitEvent(s, reader[i].cast));
+  int rc = build_clearance(V, cut, grid, s);
+  if (rc) return rc;
+  ASC_CUDA(cudaEventRecord(built, s));
+  if (capturing) ASC_CUDA(cudaStreamSynchronize(s));
+  readers = 0;
+  cutoff = cut;
+  return ASC_OK;
+}
+
+int ClearanceCache::read(cudaStream_t s, bool capturing)
+{
+  if (capturing) {
+    captured = true;
+    return ASC_OK;
+  }
+  int i = 0;
+  while (i < readers && reader[i].stream != s) ++i;
+  if (i == MAX_READERS) i = oldest++ % MAX_READERS;
+  Reader& r = reader[i];
+  if (!r.cast) ASC_CUDA(cudaEventCreateWithFlags(&r.cast, cudaEventDisableTiming));
+  // The new record stands for the old one too: stream order where s is the same
+  // stream (a wait would cost a cast of 8 us another 0.8), else a wait.  The
+  // per-thread default stream is one name of many streams.
+  if (i < readers && (r.stream != s || s == cudaStreamPerThread)) ASC_CUDA(cudaStreamWaitEvent(s, r.cast));
+  ASC_CUDA(cudaEventRecord(r.cast, s));
+  r.stream = s;
+  readers = std::max(readers, i + 1);
+  return ASC_OK;
+}
+
 int launch_filter(const asc_filter_desc& f, const float* in, float* out, int w, int h, cudaStream_t s)
 {
   if (w <= 0 || h <= 0) return ASC_OK;
@@ -1035,8 +1123,6 @@ ASC_API int asc_volume_create(const void* data, int W, int H, int D, int bps, co
       2147483648.0)
     return ASC_ERR_RANGE;
   auto* v = new asc_volume_host();
-  v->clr = nullptr;
-  v->clr_cutoff = NAN;
   int dims[3] = {mx[0] - mn[0] + 1, mx[1] - mn[1] + 1, mx[2] - mn[2] + 1};
   float norm = bps == 8 ? 255.0f : 65535.0f;
   v->min_value = vmin / norm;
@@ -1108,7 +1194,6 @@ ASC_API int asc_volume_destroy(asc_volume vol)
   if (!v) return ASC_ERR_ARG;
   Gate g(device_gate());
   cudaFree(v->pairs);
-  if (v->clr) cudaFree(v->clr);
   delete v;
   return ASC_OK;
 }
@@ -1149,21 +1234,17 @@ ASC_API int asc_raycast(asc_volume vol, const double imv[16], const float vp[4],
   }
   float m[12];
   fold_matrix(imv, v->inv_scale, v->inv_trans, m);
-  const uint8_t* clr = nullptr;
-  if (g_empty_skip) {
-    const float cut = occupancy_threshold(make_cutoff(cutoff, v->dev.norm, v->dev.gmax));
-    if (!v->clr) {
-      Gate g(device_gate());
-      ASC_CUDA(cudaMalloc(&v->clr, clearance_cells(v->dev)));
-    }
-    if (!(v->clr_cutoff == cut)) {
-      int rc = build_clearance(v->dev, cut, v->clr, S(stream));
-      if (rc) return rc;
-      v->clr_cutoff = cut;
-    }
-    clr = v->clr;
-  }
-  return raycast_launch(v->dev, clr, m, vp, step, intensity, cutoff, out, false, w, h, S(stream));
+  const float cut = occupancy_threshold(make_cutoff(cutoff, v->dev.norm, v->dev.gmax));
+  cudaStream_t s = S(stream);
+  if (!g_empty_skip)
+    return raycast_launch(v->dev, nullptr, m, vp, step, intensity, cutoff, out, false, w, h, s);
+  cudaStreamCaptureStatus capture;
+  ASC_CUDA(cudaStreamIsCapturing(s, &capture));
+  const bool capturing = capture != cudaStreamCaptureStatusNone;
+  std::lock_guard<std::mutex> lock(v->clr.mu);
+  int rc = v->clr.use(v->dev, cut, s, capturing);
+  if (!rc) rc = raycast_launch(v->dev, v->clr.grid, m, vp, step, intensity, cutoff, out, false, w, h, s);
+  return rc ? rc : v->clr.read(s, capturing);
 }
 
 // ---- images ----

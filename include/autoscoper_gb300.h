@@ -115,7 +115,10 @@ int asc_volume_destroy(asc_volume vol);
  * (RayCaster_kernels.cu:81-104).  inv_model_view: the 16 doubles of
  * CoordFrame::to_matrix_row_order of the camera->volume frame (the
  * normalisation is folded in here, as setInvModelView does);
- * viewport: (x, y, width, height) on the film plane; visible = 0 clears. */
+ * viewport: (x, y, width, height) on the film plane; visible = 0 clears.
+ * Any streams and threads may cast one volume at a time, each with its own
+ * cutoff, and casts may be captured: the volume's clearance grid, kept for the
+ * last cutoff, is built in their order. */
 int asc_raycast(asc_volume vol, const double inv_model_view[16], const float viewport[4], float sample_distance,
                 float ray_intensity, float cutoff, int visible, float *out, int width, int height, void *stream);
 

@@ -580,13 +580,17 @@ __device__ __forceinline__ BeamRay beam_ray(const float* m, const float* vp, flo
 
 // Whether the beam of all rays with directions within w (per axis) of D,
 // between t = tc - half and tc + half, may hold a sample above the threshold.
+// wide: no clearance could clear it, it reaches too far from its middle.
 __device__ __forceinline__ bool beam_occupied(const uint8_t* __restrict__ clr, int nx, int ny, int nz, const float* O,
-                                              const float* D, const float* w, float tc, float half, float err)
+                                              const float* D, const float* w, float tc, float half, float err,
+                                              bool& wide)
 {
   float h = 0.f;
   for (int i = 0; i < 3; ++i) h = fmaxf(h, fmaf(tc + half, w[i], half * fabsf(D[i])));
+  const float need = h + 1.0f + err;
+  wide = wide || need > (float)CLEAR_MAX;
   const float e = clearance_at(clr, nx, ny, nz, fmaf(tc, D[0], O[0]), fmaf(tc, D[1], O[1]), fmaf(tc, D[2], O[2]));
-  return !(e >= h + 1.0f + err);
+  return !(e >= need);
 }
 
 // The march re-bases its FP32 coordinates every REBASE samples (march_block).

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "asc_internal.cuh"
+#include "asc_clear.cuh"
 #include "asc_rays.cuh"
 
 namespace asc {
@@ -622,76 +623,27 @@ __global__ void __launch_bounds__(RB) k_hdist_sad(const float* __restrict__ f, c
   }
 }
 
-// The clearance grid (asc_march.cuh) of CB^3 cells per block.  The maximum
-// norm is separable, so the distance is taken along x, then y, then z, in
-// shared memory: a 64-bit word per row of the block's voxels and CLEAR_MAX
-// around them, a byte per (cell x, y, z), a byte per (cell x, cell y, z), and
-// the cells.  Every voxel is read (62 / 32)^3 = 7 times, from L2.
-constexpr int CB = 16;                              // cells of a block's edge
-constexpr int CV = CLEAR_CELL * CB + 2 * CLEAR_MAX;  // voxels of its edge, the surroundings included
-constexpr int CLEAR_THREADS = 512;
-constexpr size_t CLEAR_SMEM = (size_t)CV * CV * 8 + (size_t)CB * CV * CV + (size_t)CB * CB * CV;
-static_assert(CV <= 64, "a row of voxels is a 64-bit word");
-
-// min over the cell's surroundings of max(distance along the axis, d[i *
-// stride]): cell c covers entries [CLEAR_MAX + 2c, CLEAR_MAX + 2c + 2], those at distance 0.
-__device__ __forceinline__ int clear_along(const uint8_t* d, int stride, int c)
-{
-  const uint8_t* p = d + (CLEAR_MAX + CLEAR_CELL * c) * stride;
-  int e = min((int)p[0], min((int)p[stride], (int)p[2 * stride]));
-  for (int i = 1; i < CLEAR_MAX && i < e; ++i) {
-    e = min(e, max(i, (int)p[-i * stride]));
-    if (CLEAR_MAX + CLEAR_CELL * c + CLEAR_CELL + i < CV) e = min(e, max(i, (int)p[(CLEAR_CELL + i) * stride]));
-  }
-  return e;
-}
-
 template <int STORE>
 __global__ void __launch_bounds__(CLEAR_THREADS) k_clearance(DevVolume V, float cutoff_raw, uint8_t* __restrict__ clr)
 {
-  extern __shared__ unsigned long long clear_sm[];
-  unsigned long long* rows = clear_sm;               // [z][y]
-  uint8_t* dx = (uint8_t*)(rows + CV * CV);          // [z][y][cell x]
-  uint8_t* dy = dx + CB * CV * CV;                   // [z][cell y][cell x]
-  const int gx = clear_dim(V.nx), gy = clear_dim(V.ny), gz = clear_dim(V.nz);
-  const int cx0 = blockIdx.x * CB, cy0 = blockIdx.y * CB, cz0 = blockIdx.z * CB;
-  const int x0 = CLEAR_CELL * cx0 - CLEAR_MAX, y0 = CLEAR_CELL * cy0 - CLEAR_MAX, z0 = CLEAR_CELL * cz0 - CLEAR_MAX;
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x >> 5; i < CV * CV; i += CLEAR_THREADS / 32) {  // a warp per row
-    const int y = y0 + i % CV, z = z0 + i / CV;
-    unsigned long long bits = 0;
-    if (y >= 0 && y < V.ny && z >= 0 && z < V.nz)
-      for (int half = 0; half < 2; ++half) {
-        const int x = x0 + 32 * half + lane;
-        const bool above = x >= 0 && x < V.nx && 32 * half + lane < CV &&
-                           voxel_value<STORE>(V, (size_t)(z + PAD) * V.pxy + (size_t)(y + PAD) * V.px + (x + PAD)) > cutoff_raw;
-        bits |= (unsigned long long)__ballot_sync(FULL_WARP, above) << (32 * half);
-      }
-    if (lane == 0) rows[i] = bits;
-  }
+  extern __shared__ __align__(8) unsigned char clear_sm[];
+  ClearWork& w = *reinterpret_cast<ClearWork*>(clear_sm);
+  const int t = threadIdx.x, cx = blockIdx.x * CB, cy = blockIdx.y * CB, cz = blockIdx.z * CB;
+#pragma unroll 4
+  for (int i = t >> 5; i < CLEAR_Z * CLEAR_Y / 2; i += CLEAR_THREADS / 32) clear_load<STORE>(V, cutoff_raw, w, i, cx, cy, cz);
   __syncthreads();
-  for (int i = threadIdx.x; i < CB * CV * CV; i += CLEAR_THREADS) {
-    // the row's voxels from 2c - 15 on: bits 15 .. 17 are at distance 0, bit
-    // 14 - d lies d + 1 before the cell, bit 17 + d d past it
-    const unsigned long long m = rows[i / CB] >> (CLEAR_CELL * (i % CB));
-    const unsigned before = (unsigned)m & ((1u << CLEAR_MAX) - 1u);
-    const unsigned past = (unsigned)(m >> CLEAR_MAX) & ((1u << (CLEAR_MAX + CLEAR_CELL)) - 1u);
-    int e = CLEAR_MAX;
-    if (before) e = min(e, CLEAR_MAX - (31 - __clz(before)));
-    if (past) e = min(e, max(0, __ffs(past) - 1 - CLEAR_CELL));
-    dx[i] = (uint8_t)e;
+  uint2 acc = make_uint2(0u, 0u);
+  unsigned n[3] = {0u, 0u, 0u};
+#pragma unroll 1
+  for (int round = 0; CLEAR_ROUND * round <= CLEAR_REACH; ++round) {
+    clear_reach(w, t, round, acc);
+    __syncthreads();
+    clear_count(w, t, round, n);
+    __syncthreads();
   }
+  clear_bytes(w, t, n);
   __syncthreads();
-  for (int i = threadIdx.x; i < CB * CB * CV; i += CLEAR_THREADS) {
-    const int cx = i % CB, cy = i / CB % CB, z = i / (CB * CB);
-    dy[i] = (uint8_t)clear_along(dx + z * CV * CB + cx, CB, cy);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < CB * CB * CB; i += CLEAR_THREADS) {
-    const int cx = i % CB, cy = i / CB % CB, cz = i / (CB * CB);
-    if (cx0 + cx < gx && cy0 + cy < gy && cz0 + cz < gz)
-      clr[((size_t)(cz0 + cz) * gy + (cy0 + cy)) * gx + (cx0 + cx)] = (uint8_t)clear_along(dy + cy * CB + cx, CB * CB, cz);
-  }
+  clear_store(w, t, V, cx, cy, cz, clr);
 }
 
 int g_empty_skip = 1;
@@ -702,9 +654,9 @@ int build_clearance(const DevVolume& V, float cutoff_raw, uint8_t* clr, cudaStre
                       : V.storage == ASC_STORE_BF16 ? k_clearance<ASC_STORE_BF16>
                       : V.storage == ASC_STORE_F16  ? k_clearance<ASC_STORE_F16>
                                                     : k_clearance<ASC_STORE_U16>;
-  ASC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLEAR_SMEM));
+  ASC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClearWork)));
   const dim3 grid((clear_dim(V.nx) + CB - 1) / CB, (clear_dim(V.ny) + CB - 1) / CB, (clear_dim(V.nz) + CB - 1) / CB);
-  kernel<<<grid, CLEAR_THREADS, CLEAR_SMEM, s>>>(V, cutoff_raw, clr);
+  kernel<<<grid, CLEAR_THREADS, sizeof(ClearWork), s>>>(V, cutoff_raw, clr);
   ASC_LAUNCH_CHECK();
   return ASC_OK;
 }

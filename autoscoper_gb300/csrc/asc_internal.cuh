@@ -260,7 +260,10 @@ __device__ __forceinline__ void warp_sums(double (&v)[N])
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
 }
-__device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
+// step: partials from one to the next.  UNROLL: partials of a lane in flight
+// beyond the first two.
+template <int UNROLL = 1>
+__device__ __forceinline__ Moments merge_moments(const Moments* part, int nb, int step = 1)
 {
   constexpr int KEEP = 2;
   const int lane = threadIdx.x & 31;
@@ -269,7 +272,7 @@ __device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
 #pragma unroll
   for (int t = 0; t < KEEP; ++t)
 #pragma unroll
-    for (int f = 0; f < 9; ++f) kept[t][f] = lane + 32 * t < nb ? __ldcg(p + 9 * (lane + 32 * t) + f) : 0.0;
+    for (int f = 0; f < 9; ++f) kept[t][f] = lane + 32 * t < nb ? __ldcg(p + 9 * step * (lane + 32 * t) + f) : 0.0;
   double a[6] = {};  // sm, sf, sg, n and the sums of n mf, n mg
   const auto first = [&](const double* v) {
 #pragma unroll
@@ -279,11 +282,11 @@ __device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
   };
 #pragma unroll
   for (int t = 0; t < KEEP; ++t) first(kept[t]);
-#pragma unroll 1
+#pragma unroll UNROLL
   for (int i = lane + 32 * KEEP; i < nb; i += 32) {
     double v[6];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) v[f] = __ldcg(p + 9 * i + f);
+    for (int f = 0; f < 6; ++f) v[f] = __ldcg(p + 9 * step * i + f);
     first(v);
   }
   warp_sums(a);
@@ -301,11 +304,11 @@ __device__ __forceinline__ Moments merge_moments(const Moments* part, int nb)
     mg = __shfl_sync(0xffffffffu, mean, 1);
 #pragma unroll
     for (int t = 0; t < KEEP; ++t) second(kept[t]);
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int i = lane + 32 * KEEP; i < nb; i += 32) {
       double v[9];
 #pragma unroll
-      for (int f = 3; f < 9; ++f) v[f] = __ldcg(p + 9 * i + f);
+      for (int f = 3; f < 9; ++f) v[f] = __ldcg(p + 9 * step * i + f);
       second(v);
     }
     warp_sums(c);

@@ -435,11 +435,17 @@ struct ReduceScratch {
 // moments of its 4096 elements in two passes over registers, the last block
 // to finish merges all partials in FP64 and writes the correlation.  What
 // bounds it is latency: the load, two compensated block sums, then the FP64
-// tail of the last block; so a block has 1024 threads of 4 elements, each
-// block sum is finished by a warp per value, and one warp merges.  120 000
-// pixels: 31 us with 256 threads of 16 elements and a pairwise merge, 16 here.
-constexpr int NT = 1024, NE = RCHUNK / NT;
-template <int N>
+// tail of the last block.
+//
+// NT: threads per block.  1024 of 4 elements, each block sum finished by a
+// warp per value and one warp merging, where the blocks are one wave (two of
+// them on an SM): 120 000 pixels take 16 us, and 31 with 256 threads of 16
+// elements and a pairwise merge.  Beyond a wave 256 threads of 16 elements:
+// eight blocks on an SM cover one another's latencies, and the last block's
+// warps share the partials (asc_ncc_host of 2048^2 pixels: 117 us with 1024
+// threads and one warp merging, 71 here; of 4096^2: 392 and 157).  The
+// chunks, and with them the FP32 centres, are the same.
+template <int N, int NT>
 __device__ __forceinline__ void wide_sum_dfs(DFs (&v)[N], float2 (*red)[NT / 32], double* out)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -454,17 +460,33 @@ __device__ __forceinline__ void wide_sum_dfs(DFs (&v)[N], float2 (*red)[NT / 32]
   }
   __syncthreads();
   if (warp < N) {
-    const float2 p = red[warp][lane];
+    const float2 p = lane < NT / 32 ? red[warp][lane] : make_float2(0.f, 0.f);
     const double t = warp_sum_d((double)p.x + (double)p.y);
     if (lane == 0) out[warp] = t;
   }
   __syncthreads();
 }
 
+// The partials of nb blocks merged by the W warps of one, in two levels; warp
+// 0's result holds.  Writes over part[0 .. W).
+template <int W>
+__device__ __forceinline__ Moments merge_block(Moments* part, int nb)
+{
+  const int warp = threadIdx.x >> 5;
+  const Moments m = merge_moments<4>(part + warp, (nb - warp + W - 1) / W, W);
+  __syncthreads();  // every partial is read
+  if ((threadIdx.x & 31) == 0) part[warp] = m;
+  __threadfence();
+  __syncthreads();
+  return merge_moments(part, W);
+}
+
+template <int NT>
 __global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const float* __restrict__ g,
                                             const float* __restrict__ mask, unsigned n, int tree, ReduceScratch sc,
                                             double* __restrict__ result)
 {
+  constexpr int NE = RCHUNK / NT;
   __shared__ float2 red[6][NT / 32];
   __shared__ double ds[6], dc[3];
   __shared__ float s_mean[2];
@@ -504,7 +526,7 @@ __global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const f
       }
     }
   }
-  wide_sum_dfs<6>(s, red, ds);
+  wide_sum_dfs<6, NT>(s, red, ds);
   if (threadIdx.x < 2) s_mean[threadIdx.x] = ds[3] > 0 ? (float)(ds[4 + threadIdx.x] / ds[3]) : 0.f;
   __syncthreads();
   const float mf = s_mean[0], mg = s_mean[1];
@@ -517,18 +539,27 @@ __global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const f
       dfs_add_prod(c[1], b, b);
       dfs_add_prod(c[2], a, b);
     }
-  wide_sum_dfs<3>(c, red, dc);
-  if (threadIdx.x >= 32) return;
-  bool last = false;
-  tile_moments(ds, dc, mf, mg, sc.part + blockIdx.x);
-  __threadfence();
-  __syncwarp();
-  if (threadIdx.x == 0) {
-    last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
+  wide_sum_dfs<3, NT>(c, red, dc);
+  constexpr bool ONE_WARP = NT == 1024;  // merges alone
+  __shared__ bool s_last;
+  if (ONE_WARP && threadIdx.x >= 32) return;
+  if (threadIdx.x < 32) {
+    tile_moments(ds, dc, mf, mg, sc.part + blockIdx.x);
+    __threadfence();
+    __syncwarp();
+    if (threadIdx.x == 0) s_last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
   }
-  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
+  if (ONE_WARP)
+    __syncwarp();
+  else
+    __syncthreads();
+  if (!s_last) return;
   __threadfence();
-  const Moments m = merge_moments(sc.part, gridDim.x);
+  Moments m;
+  if constexpr (ONE_WARP)
+    m = merge_moments(sc.part, gridDim.x);
+  else
+    m = merge_block<NT / 32>(sc.part, gridDim.x);
   if (threadIdx.x == 0) {
     *result = moments_ncc(m);
     *sc.ticket = 0;
@@ -536,10 +567,61 @@ __global__ void __launch_bounds__(NT) k_ncc(const float* __restrict__ f, const f
 }
 
 // The launch for n elements, the same for asc_ncc and asc_ncc_noalloc.
+constexpr unsigned NCC_WAVE = 2 * 152;  // blocks of 1024 threads that run at once
 void launch_ncc(const float* f, const float* g, const float* mask, unsigned n, int tree, ReduceScratch sc,
                 double* result, cudaStream_t s)
 {
-  k_ncc<<<(unsigned)(((size_t)n + RCHUNK - 1) / RCHUNK), NT, 0, s>>>(f, g, mask, n, tree, sc, result);
+  const unsigned blocks = (unsigned)(((size_t)n + RCHUNK - 1) / RCHUNK);
+  if (blocks <= NCC_WAVE)
+    k_ncc<1024><<<blocks, 1024, 0, s>>>(f, g, mask, n, tree, sc, result);
+  else
+    k_ncc<256><<<blocks, 256, 0, s>>>(f, g, mask, n, tree, sc, result);
+}
+
+// The sums over all blocks of the N values that thread 0 holds in v, for the
+// SAD kernels: true in the last block, with the sums in its thread 0.  Up to 64
+// blocks warp 0 adds their values by itself and the other warps leave; more
+// are shared by the block's threads, whose loads one warp would wait for one
+// after the other (asc_hdist_host of 2048^2 pixels: 90 us, 48 here; of
+// 4096^2: 380 and 161).
+template <int N>
+__device__ __forceinline__ bool sum_blocks(const float (&v)[N], ReduceScratch sc, double (&sum)[N])
+{
+  __shared__ bool s_last;
+  __shared__ double s_sum[RB / 32][N];
+  const int nb = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nb > 64 ? RB / 32 : 1;
+  if (warp >= nw) return false;
+  if (threadIdx.x == 0) {
+    double* p = (double*)(sc.part + blockIdx.x);
+#pragma unroll
+    for (int k = 0; k < N; ++k) p[k] = v[k];
+    __threadfence();
+    s_last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
+  }
+  if (nw > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (!s_last) return false;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < N; ++k) sum[k] = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < nb; i += 32 * nw)
+#pragma unroll
+    for (int k = 0; k < N; ++k) sum[k] += __ldcg((const double*)(sc.part + i) + k);
+  warp_sums(sum);
+  if (nw > 1) {
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < N; ++k) s_sum[warp][k] = sum[k];
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        for (int w = 1; w < nw; ++w) sum[k] += s_sum[w][k];
+  }
+  return true;
 }
 
 // SAD ("hdist", HDist_kernels.cu:111-203): pass 1 computes the masked means
@@ -567,20 +649,10 @@ __global__ void __launch_bounds__(RB) k_hdist_means(const float* __restrict__ f,
     }
   }
   block_sum<3>(s, red);
-  if (threadIdx.x >= 32) return;
-  bool last = false;
-  if (threadIdx.x == 0) {
-    Moments p = {s[0], s[1], s[2], 0, 0, 0, 0, 0, 0};
-    sc.part[blockIdx.x] = p;
-    __threadfence();
-    last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
-  }
-  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
-  __threadfence();
-  const Moments m = merge_moments(sc.part, gridDim.x);
-  if (threadIdx.x == 0) {
-    sc.means[0] = m.sf / m.sm;
-    sc.means[1] = m.sg / m.sm;
+  double sum[3];
+  if (sum_blocks(s, sc, sum) && threadIdx.x == 0) {
+    sc.means[0] = sum[1] / sum[0];
+    sc.means[1] = sum[2] / sum[0];
     *sc.ticket = 0;
   }
 }
@@ -606,19 +678,9 @@ __global__ void __launch_bounds__(RB) k_hdist_sad(const float* __restrict__ f, c
       s[0] += fabsf((__ldg(f + i) - mF) - (__ldg(g + i) - mG));
   }
   block_sum<1>(s, red);
-  if (threadIdx.x >= 32) return;
-  bool last = false;
-  if (threadIdx.x == 0) {
-    Moments p = {s[0], 0, 0, 0, 0, 0, 0, 0, 0};
-    sc.part[blockIdx.x] = p;
-    __threadfence();
-    last = atomicAdd(sc.ticket, 1u) == gridDim.x - 1;
-  }
-  if (!__shfl_sync(FULL_WARP, (int)last, 0)) return;
-  __threadfence();
-  const Moments m = merge_moments(sc.part, gridDim.x);
-  if (threadIdx.x == 0) {
-    *result = m.sm;
+  double sum[1];
+  if (sum_blocks(s, sc, sum) && threadIdx.x == 0) {
+    *result = sum[0];
     *sc.ticket = 0;
   }
 }

@@ -759,22 +759,22 @@ __device__ __forceinline__ float contrast_px(float axy, float v, float e1, float
 __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
 
 // k_view's dynamic shared memory, in 4-byte words: 4 words that a unit's
-// reads before a buffer's first row may touch, three stage buffers of P
-// columns, the VT x VT tile, then the region's per-column and per-row radiograph
+// reads before a buffer's first row may touch, two stage buffers of P
+// columns (run_chain), the VT x VT tile, then the region's per-column and per-row radiograph
 // mapping (texel index and weight each).  halo: the larger chain's.
 __host__ __device__ constexpr int view_ex(int halo) { return (halo + 3) & ~3; }
 __host__ __device__ constexpr int view_pitch(int halo) { return VT + 2 * view_ex(halo); }
 __host__ __device__ constexpr int view_rows(int halo) { return VT + 2 * halo; }
 __host__ __device__ constexpr size_t view_tail_floats(int halo)
 {
-  return 4 + (size_t)3 * view_rows(halo) * view_pitch(halo) + (size_t)VT * VT;
+  return 4 + (size_t)2 * view_rows(halo) * view_pitch(halo) + (size_t)VT * VT;
 }
 __host__ __device__ constexpr size_t view_smem_floats(int halo)
 {
   return view_tail_floats(halo) + (size_t)2 * (view_rows(halo) + view_pitch(halo));
 }
-// the widest chain: three square stage buffers, the tile and ten words per
-// row of the region in 224 KB
+// the widest chain an engine takes: three square stage buffers, the tile and
+// ten words per row of the region in 224 KB (more than k_view needs)
 __host__ __device__ constexpr bool view_fits(int halo)
 {
   const size_t E = view_rows(halo);
@@ -905,9 +905,9 @@ __device__ __forceinline__ void six(const float* p, float* v)
   v[5] = p[4];
 }
 
-// Applies one filter from `in` to `out` over the band of the tile and `halo`
-// pixels around it; positions outside the image get 0.  `tmp` holds the
-// horizontal pass of a Gaussian/Sharpen blur, `wsh` the 1-D weights of a blur
+// Applies one filter from `in` to `out` (a blur: may be `in`) over the band of
+// the tile and `halo` pixels around it; positions outside the image get 0.
+// `tmp` holds the horizontal pass of a Gaussian/Sharpen blur, `wsh` the 1-D weights of a blur
 // of uncommon size.
 __device__ void apply_stage(const FilterDev& f, const float* in, float* out, float* tmp, float* wsh, const Region& g,
                             int halo)
@@ -1007,19 +1007,26 @@ __device__ void apply_stage(const FilterDev& f, const float* in, float* out, flo
   __syncthreads();
 }
 
-// Runs a filter chain on the first of three stage buffers of `size` floats
+// Runs a filter chain on the first of two stage buffers of `size` floats
 // each (valid on the tile and its halo H); returns the one holding the result on the tile.
+// Sobel and Contrast go from one buffer to the other; a blur's horizontal pass
+// does, and its vertical pass, which reads the stage's input at the pixel
+// itself alone, comes back into the input's.  (A third buffer would take a
+// resident block from chains of halo 13 and more, and at 22 the last but one.)
 // Not inlined: both chains of a tile run the same code, which with it fits the instruction cache.
 __device__ __noinline__ float* run_chain(const FilterDev* fl, int nf, int H, float* buf, int size, float* wsh, Region g)
 {
   int halo = H;
-  float *in = buf, *out = buf + size;
+  float *in = buf, *other = buf + size;
   for (int s = 0; s < nf; ++s) {
+    const bool blur = fl[s].kind == 3 || fl[s].kind == 4;
     halo -= fl[s].R;
-    apply_stage(fl[s], in, out, buf + 2 * size, wsh, g, halo);
-    float* t = in;
-    in = out;
-    out = t;
+    apply_stage(fl[s], in, blur ? in : other, other, wsh, g, halo);
+    if (!blur) {
+      float* t = in;
+      in = other;
+      other = t;
+    }
   }
   return in;
 }
@@ -1156,8 +1163,8 @@ __global__ void __launch_bounds__(VNT, ASC_VIEW_MINBLOCKS)
     // this view's halo lays out the shared memory
     const int H = max(V.h_drr, V.h_rad), EX = view_ex(H), P = view_pitch(H), rows = view_rows(H);
     const int size = rows * P;
-    float* buf = smem + 4;           // three stage buffers
-    float* fdrr = buf + 3 * size;  // VT x VT final DRR, then f = DRR * mask
+    float* buf = smem + 4;           // two stage buffers
+    float* fdrr = buf + 2 * size;  // VT x VT final DRR, then f = DRR * mask
     // per region column / row: the radiograph texel pair and weight of the
     // film-plane mapping (image_axis; kNoTexel where the pixel maps outside)
     int* tcx = (int*)(smem + view_tail_floats(H));

@@ -51,3 +51,26 @@ def test_counters_follow_a_queued_evaluation():
     finally:
         L.call("asc_stream_sync", s)
         L.call("asc_stream_destroy", s)
+
+
+def test_counters_follow_a_graph():
+    """An evaluation captured into a graph of the caller's leaves no event of its
+    own; after a replay and a wait the counters are its."""
+    torch = pytest.importorskip("torch")
+    sc = S.make_scene([(40, 36, 44)], 1.0, (96, 96), 1.0, filters="sobel", seed=4)
+    api.render_targets(sc)
+    eng = api.Engine(sc, max_items=8)
+    man = np.random.default_rng(3).uniform(-1, 1, (8, 6))
+    want_cost, _ = eng.eval(np.zeros(8, np.int32), man)
+    want = _counters(eng)
+    bones, mans = api.DeviceArray.from_host(np.zeros(8, np.int32)), api.DeviceArray.from_host(man)
+    cost = api.DeviceArray(8, np.float64)
+    g = torch.cuda.CUDAGraph()
+    L.call("asc_device_sync")
+    with torch.cuda.graph(g):
+        eng.eval_device(8, bones, mans, cost, torch.cuda.current_stream().cuda_stream)
+    eng.eval(np.zeros(2, np.int32), np.zeros((2, 6)))
+    g.replay()
+    torch.cuda.synchronize()
+    assert _counters(eng) == want
+    assert np.array_equal(cost.to_host(), want_cost)

@@ -476,7 +476,7 @@ __device__ __forceinline__ void warp_fill(int* __restrict__ p, int from, int to,
 // items' view tickets (views finished here count as arrived).
 // What bounds it is the latency of one FP64 chain (~70 cycles an operation).
 // One thread per (item, view) took 78 us, with two launches after it for the
-// layout and the tile map: 88 us for 4 candidates, 99 for 300; here 28 and 74.
+// layout and the tile map: 88 us for 4 candidates, 99 for 300; here 28 and 77.
 __global__ void __launch_bounds__(SETUP_THREADS) k_setup(const SceneDev* __restrict__ sc, int n_items,
                                                          const int* __restrict__ bone_in,
                                                          const double* __restrict__ manip, Bufs b,

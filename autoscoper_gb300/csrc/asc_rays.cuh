@@ -23,19 +23,19 @@
 // next_segment instead cost every other beam 2 % (14.1 -> 14.4 ms on the batch
 // below).
 //
-// What bounds it is instruction issue: 70 % of the slots, and the packed FP32
+// What bounds it is instruction issue: 74 % of the slots, and the packed FP32
 // pairs of the sample loop take two.  A beam serves its 32 rays with one byte
 // per interval and lane; rays that walked 8-voxel cells by themselves spent
 // half of their instructions on the walk.  Neighbours' segments are of nearly
-// equal length (a warp's lanes march 88 % of the samples that its slots have
+// equal length (a warp's lanes march 85 % of the samples that its slots have
 // room for), so sorting a block's segments by length, with its barriers, costs
 // more than the idle lanes do (12.6 ms against 12.2 on the batch below).
 // k_ray over 300 candidates x 2 views of 1024^2 (three bones of up to 4.8 M
-// voxels): 16.5 ms with the walk, 12.2 with beams (15.7 G and 11.0 G warp
-// instructions), 11.8 with the sample loop's unpacking split over two units
-// and no clamp in it (march_block), 11.3 with the warp met again before each
-// march (march_beam); 100 candidates of a 128^3 bone at 512^2: 2.55, 1.44,
-// 1.42 and 1.37 ms.
+// voxels): 16.5 ms with the walk (15.7 G warp instructions), 12.2 with beams,
+// 11.8 with the sample loop's unpacking split over two units and no clamp in it
+// (march_block), 11.3 with the warp met again before each march (march_beam;
+// 12.1 G); 100 candidates of a 128^3 bone at 512^2: 2.55, 1.44, 1.42 and 1.37
+// ms.
 #pragma once
 
 #include "asc_march.cuh"

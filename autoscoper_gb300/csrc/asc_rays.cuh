@@ -15,13 +15,11 @@
 //
 // A clearance answers for 15 voxels at most, so pixels of more than about three
 // voxels, or a crossing of more than 1700, leave intervals that no clearance
-// clears.  The rays of such a beam mark their own intervals, hopping from
-// clearance to clearance (ray_mask); the same march follows.  64 candidates of a
-// 320^3 bone in two views of 96^2 (4 voxels a pixel), the whole evaluation:
-// 711 us with a walk of each ray through 8-voxel cells, 1502 with the beams'
-// intervals alone (4.4 times the samples), 538 with the rays' own.  Hops inside
-// next_segment instead cost every other beam 2 % (14.1 -> 14.4 ms on the batch
-// below).
+// clears.  The rays of such a beam find their own intervals (ray_mask); the same
+// march follows.  k_ray over 64 candidates of a 320^3 bone in two views of 152^2
+// (4 voxels a pixel): 545 us with a walk of each ray through 8-voxel cells, 1588
+// with the beams' intervals alone (4 times the samples), 520 with the rays' own; of
+// a 512^3 bone at 243^2 2360, 12600 and 2340.
 //
 // What bounds it is instruction issue: 74 % of the slots, and the packed FP32
 // pairs of the sample loop take two.  A beam serves its 32 rays with one byte
@@ -70,7 +68,7 @@ struct Beam {
   unsigned long long mask;  // bit i: interval [t0 + i len, t0 + (i + 1) len) may hold samples above the cutoff
   float t0, len;
   float err;
-  bool wide;  // an interval reaches farther than a clearance answers for: each ray has intervals of its own (ray_mask)
+  bool wide;  // an interval reaches farther than a clearance answers for: each ray finds its own (ray_mask)
 };
 
 // The occupied intervals of this warp's 32 rays.  Every lane passes a pixel
@@ -139,26 +137,40 @@ __device__ __forceinline__ int clear_samples(const DevVolume& V, const uint8_t* 
   return e >= 0.f ? (int)fminf(e * r.per, 1.0e6f) + 1 : 0;
 }
 
-// The occupied intervals of this lane's ray (K samples, tf: RaySetup::tf) in a
-// wide beam: the ray hops from clearance to clearance and marks the intervals
-// in which it stands at a sample that may count.  A sample at an interval's
-// bound may be marked on either side of it: a run holds the samples within
-// rounding of its ends (next_segment).
-template <class Slots>
+// The occupied intervals of this lane's ray (tf: RaySetup::tf) in a wide beam,
+// from tests at equal distances along the beam's crossing: enough of them that
+// a clearance of half its range clears the stretch of one, and at least a test
+// per 8 samples up to one per interval.  Rays that cross few voxels are left to
+// the trims of their ends, which reach as far (SHORT): 64 candidates in two views
+// at 4 voxels a pixel, k_ray of a 160^3 bone 165 us without tests and 148 with
+// them, of a 128^3 one 107 and 115.  The tests do not wait for one another, where
+// hopping from clearance to clearance is a chain of loads: a cast of 32^2 pixels
+// of a 320^3 bone 62 us with hops, 54 with tests.  FLIGHT: loads in flight, which
+// shorten a single image (four; 58 us with two) but crowd L1 when every warp
+// marches (64 candidates of a 512^3 bone: 2.48 ms with four, 2.33 with two).
+constexpr float CLEAR_HALF = 0.5f * (CLEAR_MAX - 1);
+constexpr int SHORT = 10;  // in units of 2 CLEAR_HALF voxels
+template <int FLIGHT, class Slots>
 __device__ __forceinline__ unsigned long long ray_mask(const DevVolume& V, const uint8_t* __restrict__ clr,
                                                        const Slots& S, int K, float tf, const Beam& b)
 {
-  const ClearRay r = clear_ray(S);
-  const float per = approx_rcp(b.len);
+  const float4 q0 = S.q[0][threadIdx.x], q1 = S.q[1][threadIdx.x], q2 = S.q[2][threadIdx.x];
+  const float dX = q1.z, dY = q2.x, dZ = q2.z;
+  const float d = K > 0 ? fmaxf(fabsf(dX), fmaxf(fabsf(dY), fabsf(dZ))) : 0.f;  // voxels a sample
+  const unsigned far = __reduce_max_sync(FULL_WARP, (unsigned)fminf(b.len * d * (32.0f / CLEAR_HALF), 4096.0f));
+  if (far <= SHORT || 4.0f * (float)far > 64.0f * b.len) return ~0ull;  // a test for fewer than four samples gains nothing
+  const unsigned tests = max(far, (unsigned)fminf(8.0f * b.len, 64.0f));
+  int lt = 0;  // log2 of the tests made
+  while ((1u << lt) < tests) ++lt;
+  const float len = b.len * (lt <= 6 ? (float)(64 >> lt) : 1.0f / (float)(1 << (lt - 6)));
+  const float need = fmaf(0.5f * len, d, 1.0f + b.err);
+  const unsigned long long bits = lt <= 6 ? ~0ull >> (64 - (64 >> lt)) : 1ull;
   unsigned long long mask = 0ull;
-  for (int k = 0; k < K;) {
-    const int f = clear_samples(V, clr, r, b.err, k);
-    k += f;
-    if (f == 0) {
-      const int i = min(max((int)((tf - (float)k - b.t0) * per), 0), 63);
-      mask |= 1ull << i;
-      k = max(k, (int)floorf(tf - fmaf((float)i, b.len, b.t0))) + 1;
-    }
+#pragma unroll FLIGHT
+  for (int j = 0; j < 1 << lt; ++j) {
+    const float k = tf - fmaf((float)j + 0.5f, len, b.t0);
+    const float e = clearance_at(clr, V.nx, V.ny, V.nz, fmaf(-k, dX, q0.x), fmaf(-k, dY, q0.z), fmaf(-k, dZ, q1.x));
+    if (!(e >= need)) mask |= bits << (lt <= 6 ? j << (6 - lt) : j >> (lt - 6));
   }
   return mask;
 }
@@ -233,7 +245,7 @@ __device__ __forceinline__ float march_beam(const DevVolume& V, const uint8_t* _
                                             unsigned& marched, unsigned& slots)
 {
   RunState run{b.mask, 0, -1, 0, -1, 0};
-  if (b.wide) run.mask &= ray_mask(V, clr, S, K, fabsf(tf), b);
+  if (b.wide) run.mask &= ray_mask<2 * PAIRS>(V, clr, S, K, fabsf(tf), b);
   if (K <= 0) run.mask = 0;
   df total{0.f, 0.f};  // NaN once a segment met the cutoff's band
   for (;;) {

@@ -197,7 +197,7 @@ int mask_images(const float* drr, const float* rad, const float* bg, float* mask
 constexpr int FT = 32;  // output tile edge
 
 struct StencilArgs {
-  int kind;    // 0 contrast, 1 sobel, 3 gaussian, 4 sharpen
+  int kind;    // 0 contrast, 1 sobel (k_filter alone), 3 gaussian, 4 sharpen
   int K;       // taps per axis (gaussian / sharpen) or window (contrast)
   float p0, p1, p2;
   float g[64];
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) k_stencil(const float* __restrict__ in, f
                                                  StencilArgs a)
 {
   extern __shared__ float sm[];
-  const int R = a.kind == 1 ? 1 : (a.kind == 0 ? (a.K / 2 > (a.K - 1) / 2 ? a.K / 2 : (a.K - 1) / 2) : a.K / 2);
+  const int R = a.K / 2;
   const int E = FT + 2 * R;  // staged edge
   float* tile = sm;           // E x E
   float* hp = sm + E * E;     // E rows x FT (horizontal pass)
@@ -239,31 +239,16 @@ __global__ void __launch_bounds__(256) k_stencil(const float* __restrict__ in, f
       } else {
         r = fabsf(f - blur) > a.p2 ? fminf(fmaxf(f + a.p1 * (f - blur), 0.f), 1.f) : f;
       }
-    } else if (a.kind == 1) {
-      // Sobel with clamp-to-edge neighbours (SobelFilter_kernels.cu:69-96)
-      int xm = gx > 0 ? -1 : 0, xp = gx < w - 1 ? 1 : 0, ym = gy > 0 ? -1 : 0, yp = gy < h - 1 ? 1 : 0;
-      const float* c = tile + (ty + R) * E + tx + R;
-      float p00 = c[ym * E + xm], p01 = c[ym * E], p02 = c[ym * E + xp];
-      float p10 = c[xm], p12 = c[xp];
-      float p20 = c[yp * E + xm], p21 = c[yp * E], p22 = c[yp * E + xp];
-      float horz = p02 + 2 * p12 + p22 - p00 - 2 * p10 - p20;
-      float vert = p00 + 2 * p01 + p02 - p20 - 2 * p21 - p22;
-      float grad = sqrtf(horz * horz + vert * vert);
-      float s = a.p1 < 0.5f ? a.p0 * grad + 2.0f * a.p1 * f : 2.0f * (1.0f - a.p1) * a.p0 * grad + f;
-      r = fminf(fmaxf(s, 0.f), 1.f);
     } else {
       // Contrast: box mean over the in-image part of the window
       // (ContrastFilter_kernels.cu:64-80), then axy^(a-b) * f^b.
       int size = a.K;
       int i0 = max(gy - size / 2, 0), i1 = min(gy + (size + 1) / 2, h);
       int j0 = max(gx - size / 2, 0), j1 = min(gx + (size + 1) / 2, w);
-      float n = 0.f, s = 0.f;
+      float s = 0.f;
       for (int yy = i0; yy < i1; ++yy)
-        for (int xx = j0; xx < j1; ++xx) {
-          n += 1.0f;
-          s += tile[(yy - y0) * E + (xx - x0)];
-        }
-      float axy = s / n;
+        for (int xx = j0; xx < j1; ++xx) s += tile[(yy - y0) * E + (xx - x0)];
+      float axy = s / (float)((i1 - i0) * (j1 - j0));
       r = axy > 0.01f ? powf(axy, a.p0 - a.p1) * powf(f, a.p1) : 0.0f;
     }
     out[(size_t)gy * w + gx] = r;
